@@ -440,7 +440,7 @@ k_adjoint(const SolveParams P, const AdParams A, const double* __restrict__ tab6
     double* sJ = (double*)(smem_raw + M.jsum);
 
     const int tid = threadIdx.x;
-    const int cc = thread_col<double>(tid), g = thread_g<double>(tid);
+    const int cc = thread_col_ad(tid), g = thread_g_ad(tid);
     const int ib = cT.ngb[g], igb = cT.gib[g];
     const bool nir = ib <= 8 || ib == 13;
     const bool fused = P.fused && P.icld >= 1;

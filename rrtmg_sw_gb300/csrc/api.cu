@@ -243,7 +243,7 @@ int build_tables(State& st) {
     T.exp_tbl = put(et);
     // band/region descriptors of the FP32 gas optics (rrtmg_sw_taumol.f90:275-1785)
     enum { H2O = 0, CO2 = 1, O3 = 2, CH4 = 3, O2 = 4, O2CONT = 9 };
-    auto reg = [&](int band, int up, int kind, int sa, int sb, float strrat, float fac, int cont, int minor,
+    auto reg = [&](int band, int up, int kind, int sa, int sb, double strrat, double fac, int cont, int minor,
                    int mtab, int rtype, int rtab) {
         TmRegion& r = T.tm[band - 16][up];
         const BandOff& b = T.b[band - 16];
@@ -251,39 +251,46 @@ int build_tables(State& st) {
         r.minor = (int8_t)minor; r.rtype = (int8_t)rtype;
         r.nsp = (int8_t)(kind == 1 ? (up ? b.nspb : b.nspa) : 1);
         r.jo = (int8_t)(up ? 13 : 1);
-        r.strrat = strrat; r.fac = fac; r.mult = up ? 4.0f : 8.0f;
+        r.strrat = (float)strrat; r.fac = (float)fac; r.mult = up ? 4.0f : 8.0f;
+        T.strrat64[band - 16][up] = strrat;
+        T.fac64[band - 16][up] = fac;
         r.ktab = up ? b.absb : b.absa;
         r.mtab = mtab;
         r.rtab = rtab;
     };
-    reg(16, 0, 1, H2O, CH4, 252.131f, 1.f, 1, -1, 0, 0, T.b[16 - 16].rayl);
-    reg(16, 1, 2, CH4, 0, 0.f, 1.f, 0, -1, 0, 0, T.b[16 - 16].rayl);
-    reg(17, 0, 1, H2O, CO2, 0.364641f, 1.f, 1, -1, 0, 0, T.b[17 - 16].rayl);
-    reg(17, 1, 1, H2O, CO2, 0.364641f, 1.f, 2, -1, 0, 0, T.b[17 - 16].rayl);
-    reg(18, 0, 1, H2O, CH4, 38.9589f, 1.f, 1, -1, 0, 0, T.b[18 - 16].rayl);
-    reg(18, 1, 2, CH4, 0, 0.f, 1.f, 0, -1, 0, 0, T.b[18 - 16].rayl);
-    reg(19, 0, 1, H2O, CO2, 5.49281f, 1.f, 1, -1, 0, 0, T.b[19 - 16].rayl);
-    reg(19, 1, 2, CO2, 0, 0.f, 1.f, 0, -1, 0, 0, T.b[19 - 16].rayl);
-    reg(20, 0, 2, H2O, 0, 0.f, 1.f, 1, CH4, T.b[20 - 16].absch4, 0, T.b[20 - 16].rayl);
-    reg(20, 1, 2, H2O, 0, 0.f, 1.f, 2, CH4, T.b[20 - 16].absch4, 0, T.b[20 - 16].rayl);
-    reg(21, 0, 1, H2O, CO2, 0.0045321f, 1.f, 1, -1, 0, 0, T.b[21 - 16].rayl);
-    reg(21, 1, 1, H2O, CO2, 0.0045321f, 1.f, 2, -1, 0, 0, T.b[21 - 16].rayl);
-    reg(22, 0, 1, H2O, O2, (float)(1.6 * 0.022708), 1.f, 1, O2CONT, 0, 0, T.b[22 - 16].rayl);
-    reg(22, 1, 2, O2, 0, 0.f, 1.6f, 0, O2CONT, 0, 0, T.b[22 - 16].rayl);
-    reg(23, 0, 2, H2O, 0, 0.f, 1.029f, 1, -1, 0, 1, T.b[23 - 16].rayl);
-    reg(23, 1, 0, 0, 0, 0.f, 1.f, 0, -1, 0, 1, T.b[23 - 16].rayl);
-    reg(24, 0, 1, H2O, O2, 0.124692f, 1.f, 1, O3, T.b[24 - 16].abso3a, 2, T.b[24 - 16].rayla);
-    reg(24, 1, 2, O2, 0, 0.f, 1.f, 0, O3, T.b[24 - 16].abso3b, 1, T.b[24 - 16].raylb);
-    reg(25, 0, 2, H2O, 0, 0.f, 1.f, 0, O3, T.b[25 - 16].abso3a, 1, T.b[25 - 16].rayl);
-    reg(25, 1, 0, 0, 0, 0.f, 1.f, 0, O3, T.b[25 - 16].abso3b, 1, T.b[25 - 16].rayl);
-    reg(26, 0, 0, 0, 0, 0.f, 1.f, 0, -1, 0, 1, T.b[26 - 16].rayl);
-    reg(26, 1, 0, 0, 0, 0.f, 1.f, 0, -1, 0, 1, T.b[26 - 16].rayl);
-    reg(27, 0, 2, O3, 0, 0.f, 1.f, 0, -1, 0, 1, T.b[27 - 16].rayl);
-    reg(27, 1, 2, O3, 0, 0.f, 1.f, 0, -1, 0, 1, T.b[27 - 16].rayl);
-    reg(28, 0, 1, O3, O2, 6.67029e-07f, 1.f, 0, -1, 0, 0, T.b[28 - 16].rayl);
-    reg(28, 1, 1, O3, O2, 6.67029e-07f, 1.f, 0, -1, 0, 0, T.b[28 - 16].rayl);
-    reg(29, 0, 2, H2O, 0, 0.f, 1.f, 1, CO2, T.b[29 - 16].absco2, 0, T.b[29 - 16].rayl);
-    reg(29, 1, 2, CO2, 0, 0.f, 1.f, 0, H2O, T.b[29 - 16].absh2o, 0, T.b[29 - 16].rayl);
+    reg(16, 0, 1, H2O, CH4, 252.131, 1.0, 1, -1, 0, 0, T.b[16 - 16].rayl);
+    reg(16, 1, 2, CH4, 0, 0.0, 1.0, 0, -1, 0, 0, T.b[16 - 16].rayl);
+    reg(17, 0, 1, H2O, CO2, 0.364641, 1.0, 1, -1, 0, 0, T.b[17 - 16].rayl);
+    reg(17, 1, 1, H2O, CO2, 0.364641, 1.0, 2, -1, 0, 0, T.b[17 - 16].rayl);
+    reg(18, 0, 1, H2O, CH4, 38.9589, 1.0, 1, -1, 0, 0, T.b[18 - 16].rayl);
+    reg(18, 1, 2, CH4, 0, 0.0, 1.0, 0, -1, 0, 0, T.b[18 - 16].rayl);
+    reg(19, 0, 1, H2O, CO2, 5.49281, 1.0, 1, -1, 0, 0, T.b[19 - 16].rayl);
+    reg(19, 1, 2, CO2, 0, 0.0, 1.0, 0, -1, 0, 0, T.b[19 - 16].rayl);
+    reg(20, 0, 2, H2O, 0, 0.0, 1.0, 1, CH4, T.b[20 - 16].absch4, 0, T.b[20 - 16].rayl);
+    reg(20, 1, 2, H2O, 0, 0.0, 1.0, 2, CH4, T.b[20 - 16].absch4, 0, T.b[20 - 16].rayl);
+    reg(21, 0, 1, H2O, CO2, 0.0045321, 1.0, 1, -1, 0, 0, T.b[21 - 16].rayl);
+    reg(21, 1, 1, H2O, CO2, 0.0045321, 1.0, 2, -1, 0, 0, T.b[21 - 16].rayl);
+    reg(22, 0, 1, H2O, O2, 1.6 * 0.022708, 1.0, 1, O2CONT, 0, 0, T.b[22 - 16].rayl);
+    reg(22, 1, 2, O2, 0, 0.0, 1.6, 0, O2CONT, 0, 0, T.b[22 - 16].rayl);
+    reg(23, 0, 2, H2O, 0, 0.0, 1.029, 1, -1, 0, 1, T.b[23 - 16].rayl);
+    reg(23, 1, 0, 0, 0, 0.0, 1.0, 0, -1, 0, 1, T.b[23 - 16].rayl);
+    reg(24, 0, 1, H2O, O2, 0.124692, 1.0, 1, O3, T.b[24 - 16].abso3a, 2, T.b[24 - 16].rayla);
+    reg(24, 1, 2, O2, 0, 0.0, 1.0, 0, O3, T.b[24 - 16].abso3b, 1, T.b[24 - 16].raylb);
+    reg(25, 0, 2, H2O, 0, 0.0, 1.0, 0, O3, T.b[25 - 16].abso3a, 1, T.b[25 - 16].rayl);
+    reg(25, 1, 0, 0, 0, 0.0, 1.0, 0, O3, T.b[25 - 16].abso3b, 1, T.b[25 - 16].rayl);
+    reg(26, 0, 0, 0, 0, 0.0, 1.0, 0, -1, 0, 1, T.b[26 - 16].rayl);
+    reg(26, 1, 0, 0, 0, 0.0, 1.0, 0, -1, 0, 1, T.b[26 - 16].rayl);
+    reg(27, 0, 2, O3, 0, 0.0, 1.0, 0, -1, 0, 1, T.b[27 - 16].rayl);
+    reg(27, 1, 2, O3, 0, 0.0, 1.0, 0, -1, 0, 1, T.b[27 - 16].rayl);
+    reg(28, 0, 1, O3, O2, 6.67029e-07, 1.0, 0, -1, 0, 0, T.b[28 - 16].rayl);
+    reg(28, 1, 1, O3, O2, 6.67029e-07, 1.0, 0, -1, 0, 0, T.b[28 - 16].rayl);
+    reg(29, 0, 2, H2O, 0, 0.0, 1.0, 1, CO2, T.b[29 - 16].absco2, 0, T.b[29 - 16].rayl);
+    reg(29, 1, 2, CO2, 0, 0.0, 1.0, 0, H2O, T.b[29 - 16].absh2o, 0, T.b[29 - 16].rayl);
+    {
+        const int two[8] = {16, 17, 18, 19, 21, 22, 24, 28};
+        for (int b = 0; b < NBND; ++b) T.sslot[b] = -1;
+        for (int k = 0; k < 8; ++k) T.sslot[two[k] - 16] = (int8_t)k;
+    }
     T.total = (int)B.size();
     T.oneminus = 1.0 - 1.e-06;  // rrtmg_sw_rad.f90:563-565
     T.bpade_f = (float)T.bpade;
@@ -594,7 +601,6 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
     LaunchInfo li = fp32 ? plan_fp32(P, st.num_sms, allow_tiled && !st.no_tiled) : plan_fp64(P, st.num_sms);
     st.last_kernel = !fp32 ? RRTMG_SW_KERNEL_FP64 : li.tiled ? RRTMG_SW_KERNEL_FP32_TILED : RRTMG_SW_KERNEL_FP32;
     st.last_tile_slots = fp32 && li.tiled ? li.tile_slots : 0;
-    if (!fp32) li.slot_bytes = slot_elems(P.nlay, P.idelm, false) * sizeof(double);
     P.slot_elems = li.slot_bytes / (fp32 ? sizeof(float) : sizeof(double));
     // tiled: per-CTA areas, then the pairs' prepared blocks, then the overflow list
     const size_t off_prep = ovf_offset((size_t)li.grid * li.slot_bytes);
@@ -1054,11 +1060,12 @@ int solve_static(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cu
     if (li.tiled && off_prep + (size_t)P.npairs * li.prep_bytes > avail) li = plan_fp32(P, st.num_sms, false);
     st.last_kernel = !fp32 ? RRTMG_SW_KERNEL_FP64 : li.tiled ? RRTMG_SW_KERNEL_FP32_TILED : RRTMG_SW_KERNEL_FP32;
     st.last_tile_slots = fp32 && li.tiled ? li.tile_slots : 0;
-    if (!fp32) li.slot_bytes = slot_elems(P.nlay, P.idelm, false) * sizeof(double);
-    const size_t slots = avail / li.slot_bytes;
-    // one slot per SM, or per column pair when the call has fewer pairs
+    // one slot per SM, or per column pair when the call has fewer pairs, of
+    // the documented size (the FP64 form's own slots are smaller)
     const size_t need = (size_t)std::min(li.grid, st.num_sms);
-    if (slots < need) return RRTMG_SW_ESCRATCH;
+    const size_t doc_bytes = fp32 ? li.slot_bytes : slot_elems(P.nlay, P.idelm) * sizeof(double);
+    if (avail / doc_bytes < need) return RRTMG_SW_ESCRATCH;
+    const size_t slots = avail / li.slot_bytes;
     if ((size_t)li.grid > slots) li.grid = (int)slots;
     P.slot_elems = li.slot_bytes / (fp32 ? sizeof(float) : sizeof(double));
     StaticArea area;
@@ -1273,7 +1280,8 @@ int batch_plan(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, int 
         if (!rc && P[i].irng) rc = RRTMG_SW_EIRNG;
         if (rc) { batch_release(bp); return rc; }
         for (int k = 0; k < NTILE; ++k) {
-            slot[k] = std::max(slot[k], slot_elems(P[i].nlay, P[i].idelm, fp32, tiles[k]));
+            slot[k] = std::max(slot[k], fp32 ? slot_elems(P[i].nlay, P[i].idelm, tiles[k])
+                                             : slot_elems_fp64(P[i], tiles[k]));
             smem[k] = std::max(smem[k], fp32 ? solve_smem_fp32(P[i], tiles[k]) : solve_smem_fp64(P[i], tiles[k]));
         }
         cols += P[i].ncol;

@@ -70,6 +70,12 @@ struct DevTables {
     double heatfac, bpade, oneminus;
     float bpade_f, oneminus_f;
     TmRegion tm[NBND][2];
+    // FP64 gas optics: the descriptors' constants in FP64 and, for the bands
+    // whose k tables are interpolated in a species ratio, its slot (0-7) in
+    // the prepared blocks (-1: none; slots 1-7: the solar source is
+    // interpolated too)
+    double strrat64[NBND][2], fac64[NBND][2];
+    int8_t sslot[NBND];
     // GF(2) jump matrices of the KISS xorshift component: column j of
     // M^(2^k) at xs_jump[k][j]
     uint32_t xs_jump[32][32];

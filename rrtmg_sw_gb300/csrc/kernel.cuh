@@ -1,12 +1,12 @@
-// kernel.cuh -- the fused solve kernel (see solve.cuh for the pieces).
+// kernel.cuh -- pieces shared by the forms (setcoef, cell optics, column
+// maps) and the FP32 form's scratch-based solve kernel (see solve.cuh for the
+// pieces; fp64.cuh holds the FP64 form's kernels).
 #pragma once
 
 #include "solve.cuh"
 
 namespace rrsw {
 
-// levels buffered per reduction round of the g-point sums
-constexpr int KLEV = 4;
 // FP32 form: cells to redo in FP64 queued per column group (one int each:
 // thread << 20 | g-point << 12 | layer << 1 | cloudy); cells past the queue
 // are marked in the scratch and redone by their own thread
@@ -15,21 +15,12 @@ constexpr int REDO_QUEUE = 1024;
 // COLS_PER_CTA); sMisc holds their laytrop words, then the queue length
 constexpr int MAX_TILE_COLS = 4;
 constexpr int MISC_QN = MAX_TILE_COLS;
-constexpr int KLEV_F32 = 1;
-// (FP64 tiles of 4 columns buffer 2 levels: their shared memory then fits
-// the 137-layer case at one CTA per SM; the sums do not depend on it)
-__host__ __device__ constexpr int klev_of(size_t rsz, int nc = COLS_PER_CTA) {
-    return rsz == 4 ? KLEV_F32 : (nc > 2 ? KLEV / 2 : KLEV);
-}
 constexpr int NQ_MAX = 16;
-// g-point sums per level: fu, fd, cu, cd, fddir, cddir; the FP32 form adds
-// the absorption of the layer below the level (total, clear) for its
-// heating rates; with the extra outputs, + uvfd, uvcd, uvfddir, uvcddir,
-// nifd, nicd, nifddir, nicddir.
-template <typename R>
-__host__ __device__ constexpr int num_abs() { return sizeof(R) == 4 ? 2 : 0; }
-template <typename R>
-__host__ __device__ inline int num_q(bool extra) { return 6 + num_abs<R>() + (extra ? 8 : 0); }
+// g-point sums per level: fu, fd, cu, cd, fddir, cddir, the absorption of the
+// layer below the level (total, clear) for the heating rates; with the extra
+// outputs, + uvfd, uvcd, uvfddir, uvcddir, nifd, nicd, nifddir, nicddir.
+constexpr int QX = 8;  // first extra-output sum
+__host__ __device__ inline int num_q(bool extra) { return QX + (extra ? 8 : 0); }
 
 // scratch fields per level (pass 1 -> pass 2)
 enum { S_REFC, S_REFDC, S_TRAC, S_TRADC, S_DBTC, S_RUPC, S_RUPDC,
@@ -695,25 +686,19 @@ struct Smem {
 
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-__host__ __device__ inline Smem smem_layout(int L, int nq, bool fused, bool aer_stage, size_t rsz,
-                                            int nc = COLS_PER_CTA) {
+__host__ __device__ inline Smem smem_layout(int L, int nq, bool fused, bool aer_stage, int nc = COLS_PER_CTA) {
     const int nt = nc * NGPT;
     Smem m;
     size_t o = 0;
     m.tm = o;
-    // FP32 form: taumol descriptors first, at a fixed offset (the batch
-    // kernel fills them once and re-lays the rest out per instance)
-    if (rsz == sizeof(float)) o = align16(o + NBND * 2 * sizeof(TmSmem));
-    // FP32 form: queue of the cells to redo in FP64
-    m.rq = o;
-    if (rsz == sizeof(float)) o = align16(o + (REDO_QUEUE + nt) * sizeof(int));
+    // taumol descriptors first, at a fixed offset (the batch kernel fills
+    // them once and re-lays the rest out per instance)
+    o = align16(o + NBND * 2 * sizeof(TmSmem));
+    // queue of the cells to redo in FP64
+    m.rq = o;   o = align16(o + (REDO_QUEUE + nt) * sizeof(int));
     m.pdp = o;  o = align16(o + nc * L * sizeof(double));
-    m.coef = o; o = align16(o + nc * NFR * L * rsz);
-    m.hrf = o;
-    if (rsz == sizeof(float)) {
-        // FP32 form: heatfac / dp per layer
-        m.hrf = o; o = align16(o + nc * L * sizeof(float));
-    }
+    m.coef = o; o = align16(o + nc * NFR * L * sizeof(float));
+    m.hrf = o;  o = align16(o + nc * L * sizeof(float));  // heatfac / dp per layer
     m.pk = o;   o = align16(o + nc * L * sizeof(int));
     m.misc = o; o = align16(o + 8 * sizeof(int));  // laytrop per column [0, nc), redo queue length [MISC_QN]
     m.kc = m.ka = m.omcf = m.cld = m.seed = m.xs = m.aer = o;
@@ -721,15 +706,15 @@ __host__ __device__ inline Smem smem_layout(int L, int nq, bool fused, bool aer_
         m.kc = o;   o = align16(o + nc * L * sizeof(long long));
         m.ka = o;   o = align16(o + nc * L * sizeof(long long));
         m.omcf = o; o = align16(o + nc * L * sizeof(double));
-        m.cld = o;  o = align16(o + nc * 4 * L * rsz);
+        m.cld = o;  o = align16(o + nc * 4 * L * sizeof(float));
         m.seed = o; o = align16(o + nc * 4 * sizeof(uint32_t));
         m.xs = o;   o = align16(o + NGPT * 32 * sizeof(uint32_t));
     }
     if (aer_stage) {
-        m.aer = o;  o = align16(o + nc * 3 * NBND * L * rsz);
+        m.aer = o;  o = align16(o + nc * 3 * NBND * L * sizeof(float));
     }
-    m.red = o;  o = align16(o + klev_of(rsz, nc) * nq * nt * rsz);
-    m.flux = o; o = align16(o + nc * nq * (L + 1) * rsz);
+    m.red = o;  o = align16(o + nq * nt * sizeof(float));  // one level's sums
+    m.flux = o; o = align16(o + nc * nq * (L + 1) * sizeof(float));
     m.total = o;
     return m;
 }
@@ -738,72 +723,60 @@ __host__ __device__ inline Smem smem_layout(int L, int nq, bool fused, bool aer_
 // non-McICA path); the host sizes shared memory with the same test.
 __host__ __device__ inline bool stages_clouds(const SolveParams& P) { return (P.fused || P.nomcica) && P.icld >= 1; }
 
-template <typename R>
-__host__ __device__ inline bool stage_aerosol(int iaer) {
-    // the FP32 form converts the FP64 aerosol inputs once per (column, layer, band)
-    return sizeof(R) == 4 && iaer != 0;
-}
-
 // Shared-memory views of one CTA of nc columns for the parameters P.
-template <typename R>
 struct CtaView {
-    const TmSmem* sTm;  // [14][2] FP32 form: taumol descriptors
-    int* sRq;           // [REDO_QUEUE] FP32 form: cells to redo in FP64, then [nc*112] replay start per thread
+    const TmSmem* sTm;  // [14][2] taumol descriptors
+    int* sRq;           // [REDO_QUEUE] cells to redo in FP64, then [nc*112] replay start per thread
     double* sPdp;       // [nc][L]
-    R* sCoef;           // [nc][NFR][L]
-    float* sHrf;        // [nc][L] FP32 form: heatfac / dp
+    float* sCoef;       // [nc][NFR][L]
+    float* sHrf;        // [nc][L] heatfac / dp
     int* sPk;           // [nc][L]
     int* sMisc;         // laytrop [nc], redo queue length [MISC_QN]
     long long* sKc;     // [nc][L] McICA threshold of 1 - cldf
     long long* sKa;     // [nc][L] McICA threshold of alpha
     double* sOmcf;      // [nc][L] 1 - cldf (icld 2)
-    R* sCld;            // [nc][4][L] ciwp, clwp, rei, rel
+    float* sCld;        // [nc][4][L] ciwp, clwp, rei, rel
     uint32_t* sSeed;    // [nc][4]
     uint32_t* sXs;      // [112][32] columns of M^n
-    R* sAer;            // [nc][3][14][L] tau, ssa, asym
-    R* sRed;            // [KLEV][NQ][nc*112]
-    R* sFlux;           // [nc][NQ][L+1]
+    float* sAer;        // [nc][3][14][L] tau, ssa, asym
+    float* sRed;        // [NQ][nc*112]
+    float* sFlux;       // [nc][NQ][L+1]
 };
 
-template <typename R>
-__device__ inline CtaView<R> cta_view(unsigned char* smem_raw, const SolveParams& P, int nc = COLS_PER_CTA) {
-    const Smem M =
-        smem_layout(P.nlay, num_q<R>(P.extra != 0), stages_clouds(P), stage_aerosol<R>(P.iaer), sizeof(R), nc);
-    CtaView<R> v;
+__device__ inline CtaView cta_view(unsigned char* smem_raw, const SolveParams& P, int nc = COLS_PER_CTA) {
+    const Smem M = smem_layout(P.nlay, num_q(P.extra != 0), stages_clouds(P), P.iaer != 0, nc);
+    CtaView v;
     v.sTm = (const TmSmem*)(smem_raw + M.tm);
     v.sRq = (int*)(smem_raw + M.rq);
     v.sPdp = (double*)(smem_raw + M.pdp);
-    v.sCoef = (R*)(smem_raw + M.coef);
+    v.sCoef = (float*)(smem_raw + M.coef);
     v.sHrf = (float*)(smem_raw + M.hrf);
     v.sPk = (int*)(smem_raw + M.pk);
     v.sMisc = (int*)(smem_raw + M.misc);
     v.sKc = (long long*)(smem_raw + M.kc);
     v.sKa = (long long*)(smem_raw + M.ka);
     v.sOmcf = (double*)(smem_raw + M.omcf);
-    v.sCld = (R*)(smem_raw + M.cld);
+    v.sCld = (float*)(smem_raw + M.cld);
     v.sSeed = (uint32_t*)(smem_raw + M.seed);
     v.sXs = (uint32_t*)(smem_raw + M.xs);
-    v.sAer = (R*)(smem_raw + M.aer);
-    v.sRed = (R*)(smem_raw + M.red);
-    v.sFlux = (R*)(smem_raw + M.flux);
+    v.sAer = (float*)(smem_raw + M.aer);
+    v.sRed = (float*)(smem_raw + M.red);
+    v.sFlux = (float*)(smem_raw + M.flux);
     return v;
 }
 
-// FP32 form: the taumol descriptors of every band and region into shared
-// memory (offset 0 of the dynamic area); read after the next barrier.
-template <typename R>
+// The taumol descriptors of every band and region into shared memory (offset
+// 0 of the dynamic area); read after the next barrier.
 __device__ inline void fill_tm(unsigned char* smem_raw) {
-    if constexpr (sizeof(R) == 4) {
-        TmSmem* d = (TmSmem*)smem_raw;
-        for (int i = threadIdx.x; i < NBND * 2; i += blockDim.x) {
-            TmSmem t;
-            t.r = cT.tm[i / 2][i % 2];
-            t.selfref = cT.b[i / 2].selfref;
-            t.forref = cT.b[i / 2].forref;
-            t.ng = cT.b[i / 2].ng;
-            t.pad = 0;
-            d[i] = t;
-        }
+    TmSmem* d = (TmSmem*)smem_raw;
+    for (int i = threadIdx.x; i < NBND * 2; i += blockDim.x) {
+        TmSmem t;
+        t.r = cT.tm[i / 2][i % 2];
+        t.selfref = cT.b[i / 2].selfref;
+        t.forref = cT.b[i / 2].forref;
+        t.ng = cT.b[i / 2].ng;
+        t.pad = 0;
+        d[i] = t;
     }
 }
 
@@ -820,22 +793,13 @@ __device__ inline KissJump kiss_setup(const SolveParams& P, uint32_t* sXs, int g
     return J;
 }
 
-// Column slot and g-point of solve-CTA thread t.  The FP64 forms (taumol_g
-// runs a different FP64 code path per band) use warps of whole bands from
-// two columns (cT.thr_cg over each 224 threads, columns 2k and 2k+1:
-// 2200 -> 1750 ms at 262 144 x 60); the FP32 form (one descriptor-driven
-// taumol path, but cloudy layers that differ by column) is faster with 32
-// consecutive g-points of one column per warp.
-template <typename R>
-__device__ inline int thread_col(int t) {
-    if constexpr (sizeof(R) == 4) return t / NGPT;
-    else return 2 * (t / (2 * NGPT)) + (cT.thr_cg[t % (2 * NGPT)] >> 7);
-}
-template <typename R>
-__device__ inline int thread_g(int t) {
-    if constexpr (sizeof(R) == 4) return t % NGPT;
-    else return cT.thr_cg[t % (2 * NGPT)] & 127;
-}
+// Column slot and g-point of CTA thread t.  The adjoint (taumol_g runs a
+// different code path per band, in FP64 duals) uses warps of whole bands from
+// two columns (cT.thr_cg over 224 threads); the solves (one
+// descriptor-driven taumol path, but cloudy layers that differ by column) are
+// faster with 32 consecutive g-points of one column per warp.
+__device__ inline int thread_col_ad(int t) { return cT.thr_cg[t] >> 7; }
+__device__ inline int thread_g_ad(int t) { return cT.thr_cg[t] & 127; }
 
 // Column of slot c2 of column group `pair` (nc columns): consecutive
 // columns, or through the sunlit-column list of a batch (P.colmap, nmapped
@@ -848,15 +812,16 @@ __device__ inline int pair_col(const SolveParams& P, int pair, int c2, int nmapp
 
 // One group of NC columns (a column pair in the single-call kernels): prep,
 // pass 1, pass 2 and outputs, NC x 112 threads.
-template <typename R, bool MT = false, int NC = COLS_PER_CTA>
-__device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const CtaView<R>& V, const KissJump& J,
-                                           R* scr, const R* __restrict__ tab, const double* __restrict__ tab64) {
+template <bool MT = false, int NC = COLS_PER_CTA>
+__device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const CtaView& V, const KissJump& J,
+                                           float* scr, const float* __restrict__ tab,
+                                           const double* __restrict__ tab64) {
+    typedef float R;
     const int L = P.nlay;
-    const int NQ = num_q<R>(P.extra != 0);
-    constexpr int QX = 6 + num_abs<R>();  // first extra-output sum
+    const int NQ = num_q(P.extra != 0);
     const bool fused = P.fused && P.icld >= 1;
     const bool nomc = P.nomcica && P.icld >= 1;
-    const bool aer_stage = stage_aerosol<R>(P.iaer);
+    const bool aer_stage = P.iaer != 0;
     double* sPdp = V.sPdp;
     R* sCoef = V.sCoef;
     float* sHrf = V.sHrf;
@@ -872,9 +837,9 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
     R* sRed = V.sRed;
     R* sFlux = V.sFlux;
     constexpr int NT = NC * NGPT;
-    static_assert(NC % 2 == 0 && NC <= MAX_TILE_COLS, "column pairs (the FP64 thread map), up to MAX_TILE_COLS");
+    static_assert(NC % 2 == 0 && NC <= MAX_TILE_COLS, "column pairs, up to MAX_TILE_COLS");
     const int tid = threadIdx.x;
-    const int cc = thread_col<R>(tid), g = thread_g<R>(tid);
+    const int cc = tid / NGPT, g = tid % NGPT;
     const int ib = cT.ngb[g], igb = cT.gib[g];
     const bool uv = ib >= 9 && ib <= 12;  // bands 25-28 (spcvmc:629)
     const int NS = P.idelm == 0 ? NS_MAX : S_DBTCN;
@@ -882,17 +847,13 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
     const int nmapped = P.colmap ? *P.mapcount : 0;
     (void)nomc;
     __syncthreads();
-    // ---------------- prep: one (column, layer) per item; FP64 in the FP64
-    // form, FP32 with the FP64 form's indices in the FP32 form
+    // ---------------- prep: one (column, layer) per item, FP32 with the FP64
+    // form's indices
     for (int it = tid; it < NC * L; it += NT) {
         const int c2 = it / L, lay = it % L + 1;
         const int pcol = pair_col(P, pair, c2, nmapped, NC);
-        constexpr bool f32 = sizeof(R) == 4;
-        if constexpr (f32)
-            prep_layer_f32(P, pcol, lay, sCoef + c2 * NFR * L, sPk + c2 * L, sPdp + c2 * L, L, tab, tab64);
-        else
-            prep_layer<R>(P, pcol, lay, sCoef + c2 * NFR * L, sPk + c2 * L, sPdp + c2 * L, L, tab64);
-        if (f32) sHrf[c2 * L + lay - 1] = (float)(cT.heatfac / sPdp[c2 * L + lay - 1]);
+        prep_layer_f32(P, pcol, lay, sCoef + c2 * NFR * L, sPk + c2 * L, sPdp + c2 * L, L, tab, tab64);
+        sHrf[c2 * L + lay - 1] = (float)(cT.heatfac / sPdp[c2 * L + lay - 1]);
         const bool real = pcol < P.ncol;
         const size_t kl = (size_t)pcol + n * (size_t)(lay - 1);
         if (fused) {
@@ -952,7 +913,7 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
         int lt = 0;
         for (int i = 0; i < L; ++i) lt += (sPk[cc * L + i] >> 30) & 1;
         sMisc[cc] = lt;
-        if (cc == 0) sMisc[MISC_QN] = 0;  // FP32 form: redo queue length
+        if (cc == 0) sMisc[MISC_QN] = 0;  // redo queue length
     }
     __syncthreads();
     const int col = pair_col(P, pair, cc, nmapped, NC);
@@ -974,9 +935,7 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
         albp = (R)(nir ? P.aldir[col] : P.asdir[col]);
         albd = (R)(nir ? P.aldif[col] : P.asdif[col]);
         // zincflx = adjflux * ssi * prmu0 (spcvmc:349-356)
-        R src;
-        if constexpr (sizeof(R) == 4) src = solar_source_generic(ib, igb, C, P, tab, V.sTm);
-        else src = solar_source<R>(ib, igb, C, P, tab);
+        const R src = solar_source_generic(ib, igb, C, P, tab, V.sTm);
         zinc = R(P.adjflux[ib]) * src * (R)cossza;
         if (fused)
             mc.start(kiss_start(sSeed + cc * 4, J, sXs + g * 32), P.icld,
@@ -988,18 +947,16 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
 
     // ---------------- pass 1: bottom -> top
     R rupc_b = albp, rupdc_b = albd, rup_b = albp, rupd_b = albd;
-    int redo_from = L + 1;  // FP32 form: lowest layer to redo in FP64
+    int redo_from = L + 1;  // lowest layer to redo in FP64
     for (int lay = 1; lay <= L; ++lay) {
         const int jk = L + 1 - lay;
         R* sv = scr + (size_t)(jk - 1) * NS * NT + tid;
         if (!active) continue;
         R taug, taur;
-        if constexpr (sizeof(R) == 4) {
+        {
             int js;
             float fs;
             taumol_generic(ib, igb, lay, C, tab, V.sTm, taug, taur, js, fs);
-        } else {
-            taumol_g<R>(ib, igb, lay, C, tab, taug, taur);
         }
         CellIn<R> ci;
         ci.taug = taug;
@@ -1019,21 +976,18 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
         cloud_in<R>(P, col, g, lay, ib, fused, cloudy, cld, ci, tab);
         const R hrs = zinc * sHrf[cc * L + lay - 1];
         const CellOpt<R> co = cell_optics<R>(ci, P.idelm, prmu0, tab, tab64, hrs, (float)zinc);
-        // FP32 form: a table entry, the conservative switch or the
-        // resonance of this cell is too close to call in FP32; it is
+        // A table entry, the conservative switch or the resonance of this cell is too close to call in FP32; it is
         // queued and redone after this pass as the FP64 form does (a cell
         // past the queue's end is marked in the scratch instead, S_DBTC < 0,
         // -2 if cloudy, and redone by its own thread)
         int redo = 0;
-        if constexpr (sizeof(R) == 4) {
-            if (co.risky) {
-                const int qi = atomicAdd(sMisc + MISC_QN, 1);
-                if (qi < REDO_QUEUE) {
-                    V.sRq[qi] = (tid << 20) | (g << 12) | (lay << 1) | (ci.cloudy ? 1 : 0);
-                } else {
-                    redo = ci.cloudy ? 2 : 1;
-                    if (lay < redo_from) redo_from = lay;
-                }
+        if (co.risky) {
+            const int qi = atomicAdd(sMisc + MISC_QN, 1);
+            if (qi < REDO_QUEUE) {
+                V.sRq[qi] = (tid << 20) | (g << 12) | (lay << 1) | (ci.cloudy ? 1 : 0);
+            } else {
+                redo = ci.cloudy ? 2 : 1;
+                if (lay < redo_from) redo_from = lay;
             }
         }
         const RT<R>& rc = co.rc;
@@ -1058,26 +1012,25 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
             rup_b = rup;
             rupd_b = rupd;
         }
-        // the FP32 form keeps the absorptances in the transmittance slots
-        // and rebuilds ptra = 1 - pref - adir, ptrad = 1 - prefd - adif
-        constexpr bool keep_abs = sizeof(R) == 4;
+        // the transmittance slots hold the absorptances, from which pass 2
+        // rebuilds ptra = 1 - pref - adir, ptrad = 1 - prefd - adif
         sv[S_REFC * NT] = rc.ref;
         sv[S_REFDC * NT] = rc.refd;
-        sv[S_TRAC * NT] = keep_abs ? rc.adir : rc.tra;
-        sv[S_TRADC * NT] = keep_abs ? rc.adif : rc.trad;
+        sv[S_TRAC * NT] = rc.adir;
+        sv[S_TRADC * NT] = rc.adif;
         sv[S_DBTC * NT] = redo ? -(R)redo : zdbtc;
         sv[S_RUPC * NT] = rupc_b;
         sv[S_RUPDC * NT] = rupdc_b;
         sv[S_REF * NT] = rt.ref;
         sv[S_REFD * NT] = rt.refd;
-        sv[S_TRA * NT] = keep_abs ? rt.adir : rt.tra;
-        sv[S_TRAD * NT] = keep_abs ? rt.adif : rt.trad;
+        sv[S_TRA * NT] = rt.adir;
+        sv[S_TRAD * NT] = rt.adif;
         sv[S_DBT * NT] = zdbt;
         sv[S_RUP * NT] = rup_b;
         sv[S_RUPD * NT] = rupd_b;
     }
 
-    if constexpr (sizeof(R) == 4) {
+    {
         // the queued cells, one per thread across the CTA, so the FP64 work
         // of a warp is dense; a redone cell that differs from its FP32 values
         // replaces them, and its thread goes over its up-sweep again from
@@ -1092,7 +1045,7 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
         }
         for (int i = tid; i < nq; i += NT) {
             const int e = V.sRq[i];
-            const int t = e >> 20, c2 = thread_col<float>(t), gg = (e >> 12) & 127, lay = (e >> 1) & 2047;
+            const int t = e >> 20, c2 = t / NGPT, gg = (e >> 12) & 127, lay = (e >> 1) & 2047;
             const int pcol = pair_col(P, pair, c2, nmapped, NC);
             Coef64At b;
             const Coef<double> Cq = coef64_at(P, pcol, lay, sMisc[c2], tab64, b);
@@ -1115,8 +1068,8 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
     R tdbtc = R(1), tdnc = R(1), rdndc = R(0);
     R tdbt = R(1), tdn = R(1), rdnd = R(0);
     R tdbtcn = R(1), tdbtn = R(1);
-    // FP32 form: absorption of the layer above the current level, less
-    // the part that its lower face's upward flux still has to add
+    // absorption of the layer above the current level, less the part
+    // that its lower face's upward flux still has to add
     R absc = R(0), abst = R(0), adifc_up = R(0), adift_up = R(0);
     for (int jk = 1; jk <= L + 1; ++jk) {
         R q[NQ_MAX];
@@ -1134,23 +1087,19 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
             ref = sv[S_REF * NT]; refd = sv[S_REFD * NT];
             tra = sv[S_TRA * NT]; trad = sv[S_TRAD * NT];
             dbt = sv[S_DBT * NT];
-            if constexpr (sizeof(R) == 4) {
-                adirc = trac; adifc = tradc; adirt = tra; adift = trad;
-                trac = R(1) - refc - adirc;
-                tradc = R(1) - refdc - adifc;
-                tra = R(1) - ref - adirt;
-                trad = R(1) - refd - adift;
-            }
+            adirc = trac; adifc = tradc; adirt = tra; adift = trad;
+            trac = R(1) - refc - adirc;
+            tradc = R(1) - refdc - adifc;
+            tra = R(1) - ref - adirt;
+            trad = R(1) - refd - adift;
             rup = sv[S_RUP * NT]; rupd = sv[S_RUPD * NT];
             if (P.idelm == 0) { dbtcn = sv[S_DBTCN * NT]; dbtn = sv[S_DBTN * NT]; }
-            if constexpr (sizeof(R) == 4) {
-                // the next level's fields into L1 while this level computes and
-                // reduces (the level barriers keep its loads from moving up)
-                if (jk < L) {
-                    const R* nx = sv + (size_t)NS * NT;
+            // the next level's fields into L1 while this level computes and
+            // reduces (the level barriers keep its loads from moving up)
+            if (jk < L) {
+                const R* nx = sv + (size_t)NS * NT;
 #pragma unroll
-                    for (int f = 0; f < S_DBTCN; ++f) asm volatile("prefetch.global.L1 [%0];" ::"l"(nx + f * NT));
-                }
+                for (int f = 0; f < S_DBTCN; ++f) asm volatile("prefetch.global.L1 [%0];" ::"l"(nx + f * NT));
             }
         } else {
             rupc = albp; rupdc = albd; rup = albp; rupd = albd;
@@ -1165,17 +1114,15 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
             const R fu = (tdbt * rup + (tdn - tdbt) * rupd) * zrt;
             const R fdif = (tdn - tdbt + tdbt * rup * rdnd) * zrt;
             const R fd = tdbt + fdif;
-            if constexpr (sizeof(R) == 4) {
-                // layer jk-1 absorbs what enters it: the direct and diffuse
-                // beams at its top (kept from the previous level) and the
-                // upward flux at its bottom face, this level
-                q[6] = zinc * (abst + fu * adift_up);
-                q[7] = zinc * (absc + cu * adifc_up);
-                abst = tdbt * adirt + fdif * adift;
-                absc = tdbtc * adirc + cdif * adifc;
-                adift_up = adift;
-                adifc_up = adifc;
-            }
+            // layer jk-1 absorbs what enters it: the direct and diffuse
+            // beams at its top (kept from the previous level) and the
+            // upward flux at its bottom face, this level
+            q[6] = zinc * (abst + fu * adift_up);
+            q[7] = zinc * (absc + cu * adifc_up);
+            abst = tdbt * adirt + fdif * adift;
+            absc = tdbtc * adirc + cdif * adifc;
+            adift_up = adift;
+            adifc_up = adifc;
             const R dirf = P.idelm == 0 ? tdbtn : tdbt;
             const R dirc = P.idelm == 0 ? tdbtcn : tdbtc;
             q[0] = zinc * fu;
@@ -1204,45 +1151,36 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
                 tdbtn = dbtn * tdbtn;
             }
         }
-        constexpr int KL = klev_of(sizeof(R), NC);
-        const int slot = (jk - 1) % KL;
 #pragma unroll
         for (int i = 0; i < NQ_MAX; ++i)
-            if (i < NQ) sRed[(slot * NQ + i) * NT + cc * NGPT + g] = q[i];
-        if (slot == KL - 1 || jk == L + 1) {
+            if (i < NQ) sRed[i * NT + cc * NGPT + g] = q[i];
+        {
             __syncthreads();
-            const int nlev = slot + 1;
-            const int items = NC * NQ * nlev;
+            const int items = NC * NQ;
             for (int base = 0; base < items * 4; base += NT) {
                 const int t = base + tid;
                 const int item = t >> 2, part = t & 3;
                 R v = R(0);
-                int c2 = 0, qi = 0, s = 0;
+                int c2 = 0, qi = 0;
                 if (item < items) {
-                    c2 = item / (NQ * nlev);
-                    qi = (item / nlev) % NQ;
-                    s = item % nlev;
-                    const R* src = sRed + (s * NQ + qi) * NT + c2 * NGPT + part * 28;
+                    c2 = item / NQ;
+                    qi = item % NQ;
+                    const R* src = sRed + qi * NT + c2 * NGPT + part * 28;
                     for (int j = 0; j < 28; ++j) v += src[j];
                 }
                 warp_sum4(v);
-                if (item < items && part == 0) {
-                    const int jl = jk - slot + s;  // level (1 = top)
-                    sFlux[(c2 * NQ + qi) * (L + 1) + (L + 1 - jl)] = v;
-                }
+                if (item < items && part == 0) sFlux[(c2 * NQ + qi) * (L + 1) + (L + 1 - jk)] = v;
             }
             if (P.bands) {
                 // per-band sums of fu, fd, fddir, cu, cd (spcvmc:619-630 per band)
-                const int bitems = NC * NBND * 5 * nlev;
-                for (int t = tid; t < bitems; t += NT) {
-                    const int s = t % nlev, qs = (t / nlev) % 5, b = (t / (nlev * 5)) % NBND;
-                    const int c2 = t / (nlev * 5 * NBND);
+                for (int t = tid; t < NC * NBND * 5; t += NT) {
+                    const int qs = t % 5, b = (t / 5) % NBND, c2 = t / (5 * NBND);
                     const int qi = qs == 0 ? 0 : qs == 1 ? 1 : qs == 2 ? 4 : qs == 3 ? 2 : 3;
-                    const R* src = sRed + (s * NQ + qi) * NT + c2 * NGPT + cT.b[b].g0;
+                    const R* src = sRed + qi * NT + c2 * NGPT + cT.b[b].g0;
                     R v = R(0);
                     for (int j = 0; j < cT.b[b].ng; ++j) v += src[j];
                     const int ocol = pair_col(P, pair, c2, nmapped, NC);
-                    const int l = L + 1 - (jk - slot + s);  // level index, 0 = surface
+                    const int l = L + 1 - jk;  // level index, 0 = surface
                     if (ocol < P.ncol && P.bout[qs])
                         P.bout[qs][(size_t)ocol + n * ((size_t)l + (size_t)(L + 1) * b)] = (double)v;
                 }
@@ -1269,16 +1207,9 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
             double hr = 0.0, hrc = 0.0;
             if (l < L - 1) {
                 const double zdpgcp = cT.heatfac / pdp[l];
-                if constexpr (sizeof(R) == 4) {
-                    // summed layer absorption (= net-flux divergence)
-                    hr = (double)F[6 * (L + 1) + l] * zdpgcp;
-                    hrc = (double)F[7 * (L + 1) + l] * zdpgcp;
-                } else {
-                    const double fu1 = (double)F[0 * (L + 1) + l + 1], fd1 = (double)F[1 * (L + 1) + l + 1];
-                    const double cu1 = (double)F[2 * (L + 1) + l + 1], cd1 = (double)F[3 * (L + 1) + l + 1];
-                    hrc = DM(DS(DS(cd1, cu1), DS(cd, cu)), zdpgcp);
-                    hr = DM(DS(DS(fd1, fu1), DS(fd, fu)), zdpgcp);
-                }
+                // summed layer absorption (= net-flux divergence)
+                hr = (double)F[6 * (L + 1) + l] * zdpgcp;
+                hrc = (double)F[7 * (L + 1) + l] * zdpgcp;
             }
             P.swhr[o] = hr;
             P.swhrc[o] = hrc;
@@ -1296,21 +1227,21 @@ __device__ __forceinline__ void solve_pair(const SolveParams& P, int pair, const
 
 }
 
-// FP32 form: 4 resident CTAs per SM (72 registers, ~41 KB shared memory each
+// 4 resident CTAs per SM (72 registers, ~41 KB shared memory each
 // at 60 layers, level sums reduced level by level) hide more latency than 3
 // CTAs with 80 registers and 4-level reductions (147 -> 128 ms at
 // 262 144 x 60) or 2 with 128 registers.
 // MT: fused McICA from the call's MT19937 stream (P.mt) instead of KISS.
-template <typename R, bool MT>
-__global__ void __launch_bounds__(CTA_THREADS, sizeof(R) == 4 ? 4 : 2)
-k_solve(const SolveParams P, const R* __restrict__ tab, const double* __restrict__ tab64) {
+template <bool MT>
+__global__ void __launch_bounds__(CTA_THREADS, 4)
+k_solve(const SolveParams P, const float* __restrict__ tab, const double* __restrict__ tab64) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    fill_tm<R>(smem_raw);
-    const CtaView<R> V = cta_view<R>(smem_raw, P);
-    const KissJump J = kiss_setup(P, V.sXs, thread_g<R>(threadIdx.x));  // once per launch
-    R* scr = (R*)P.scratch + (size_t)blockIdx.x * P.slot_elems;
+    fill_tm(smem_raw);
+    const CtaView V = cta_view(smem_raw, P);
+    const KissJump J = kiss_setup(P, V.sXs, threadIdx.x % NGPT);  // once per launch
+    float* scr = (float*)P.scratch + (size_t)blockIdx.x * P.slot_elems;
     for (int pair = blockIdx.x; pair < P.npairs; pair += gridDim.x)
-        solve_pair<R, MT>(P, pair, V, J, scr, tab, tab64);
+        solve_pair<MT>(P, pair, V, J, scr, tab, tab64);
 }
 
 // ------------------------------------------------------------------ batch
@@ -1322,15 +1253,15 @@ k_solve(const SolveParams P, const R* __restrict__ tab, const double* __restrict
 // CTA moves to a new instance.  NC (2 or 4) is the tile the batch planner
 // picks by timing.
 
-template <typename R, int NC>
+template <int NC>
 __global__ void __launch_bounds__(NC * NGPT, 4 / NC)
 k_solve_batch(const SolveParams* __restrict__ Pb, int ninst, const int* __restrict__ counts,
-              const R* __restrict__ tab, const double* __restrict__ tab64) {
+              const float* __restrict__ tab, const double* __restrict__ tab64) {
     constexpr int NT = NC * NGPT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_pref[MAX_BATCH + 1];
     __shared__ __align__(16) SolveParams sP;
-    fill_tm<R>(smem_raw);
+    fill_tm(smem_raw);
     if (threadIdx.x == 0) {
         s_pref[0] = 0;
         for (int i = 0; i < ninst; ++i) s_pref[i + 1] = s_pref[i] + (counts[i] + NC - 1) / NC;
@@ -1338,7 +1269,7 @@ k_solve_batch(const SolveParams* __restrict__ Pb, int ninst, const int* __restri
     __syncthreads();
     const int total = s_pref[ninst];
     int cur = -1;
-    CtaView<R> V{};
+    CtaView V{};
     KissJump J{1u, 0u, 1u, 1u};
     for (int item = blockIdx.x; item < total; item += gridDim.x) {
         int lo = 0, hi = ninst;
@@ -1355,12 +1286,12 @@ k_solve_batch(const SolveParams* __restrict__ Pb, int ninst, const int* __restri
                 for (int w = threadIdx.x; w < (int)(sizeof(SolveParams) / sizeof(int)); w += NT) dst[w] = src[w];
             }
             __syncthreads();
-            V = cta_view<R>(smem_raw, sP, NC);
-            J = kiss_setup(sP, V.sXs, thread_g<R>(threadIdx.x));
+            V = cta_view(smem_raw, sP, NC);
+            J = kiss_setup(sP, V.sXs, threadIdx.x % NGPT);
             cur = lo;
         }
-        R* scr = (R*)sP.scratch + (size_t)blockIdx.x * sP.slot_elems;
-        solve_pair<R, false, NC>(sP, item - s_pref[lo], V, J, scr, tab, tab64);
+        float* scr = (float*)sP.scratch + (size_t)blockIdx.x * sP.slot_elems;
+        solve_pair<false, NC>(sP, item - s_pref[lo], V, J, scr, tab, tab64);
     }
 }
 

@@ -53,8 +53,11 @@ size_t adjoint_slot_elems(int nlay, int store);
 int adjoint_grid(const SolveParams& P, int num_sms);
 cudaError_t launch_adjoint(const SolveParams& P, const AdParams& A, const double* tab64, int num_sms, int* grid_out,
                            cudaStream_t s);
-// scratch elements (of the form's type) per CTA slot of nc columns
-size_t slot_elems(int nlay, int idelm, bool fp32, int nc = COLS_PER_CTA);
+// scratch elements per CTA slot of nc columns: of the scratch-based kernels'
+// type (also the size by which rrtmg_sw_static_dev_c refuses a call in either
+// form), and doubles of the FP64 form (fewer than the former)
+size_t slot_elems(int nlay, int idelm, int nc = COLS_PER_CTA);
+size_t slot_elems_fp64(const SolveParams& P, int nc = COLS_PER_CTA);
 
 // setcoef_sw indices of every (column, layer) through the solve's prep_layer:
 // cf (ncol x NFR x nlay), pk and pdp (ncol x nlay), column-major by column

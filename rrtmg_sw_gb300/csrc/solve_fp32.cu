@@ -213,9 +213,8 @@ LaunchInfo plan_fp32(const SolveParams& P, int num_sms, bool allow_tiled) {
         if (li.prep_grid < 1) li.prep_grid = 1;
         return li;
     }
-    li.smem = smem_layout(P.nlay, num_q<float>(P.extra != 0), stages_clouds(P),
-                          stage_aerosol<float>(P.iaer), sizeof(float)).total;
-    const auto kern = P.mt ? k_solve<float, true> : k_solve<float, false>;
+    li.smem = smem_layout(P.nlay, num_q(P.extra != 0), stages_clouds(P), P.iaer != 0).total;
+    const auto kern = P.mt ? k_solve<true> : k_solve<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)li.smem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CTA_THREADS, li.smem);
@@ -223,7 +222,7 @@ LaunchInfo plan_fp32(const SolveParams& P, int num_sms, bool allow_tiled) {
     li.grid = num_sms * per_sm;
     if (li.grid > P.npairs) li.grid = P.npairs;
     if (li.grid < 1) li.grid = 1;
-    li.slot_bytes = slot_elems(P.nlay, P.idelm, true) * sizeof(float);
+    li.slot_bytes = slot_elems(P.nlay, P.idelm) * sizeof(float);
     return li;
 }
 
@@ -234,19 +233,18 @@ cudaError_t launch_solve_fp32(const SolveParams& P, const float* tab, const doub
         else k_tiled_prep<false><<<li.prep_grid, CTA_THREADS, li.prep_smem, s>>>(P, tab, tab64);
         k_solve_tiled<<<li.grid, T_THREADS, li.smem, s>>>(P, tab, tab64);
     } else {
-        if (P.mt) k_solve<float, true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab64);
-        else k_solve<float, false><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab64);
+        if (P.mt) k_solve<true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab64);
+        else k_solve<false><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab64);
     }
     return cudaGetLastError();
 }
 
 size_t solve_smem_fp32(const SolveParams& P, int nc) {
-    return smem_layout(P.nlay, num_q<float>(P.extra != 0), stages_clouds(P), stage_aerosol<float>(P.iaer),
-                       sizeof(float), nc).total;
+    return smem_layout(P.nlay, num_q(P.extra != 0), stages_clouds(P), P.iaer != 0, nc).total;
 }
 
 int batch_blocks_per_sm_fp32(size_t smem, int nc) {
-    const auto kern = nc == 4 ? k_solve_batch<float, 4> : k_solve_batch<float, 2>;
+    const auto kern = nc == 4 ? k_solve_batch<4> : k_solve_batch<2>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nc * NGPT, smem);
@@ -255,8 +253,8 @@ int batch_blocks_per_sm_fp32(size_t smem, int nc) {
 
 cudaError_t launch_batch_fp32(const SolveParams* dPb, int n, const int* counts, const float* tab,
                               const double* tab64, int grid, size_t smem, int nc, cudaStream_t s) {
-    if (nc == 4) k_solve_batch<float, 4><<<grid, 4 * NGPT, smem, s>>>(dPb, n, counts, tab, tab64);
-    else k_solve_batch<float, 2><<<grid, 2 * NGPT, smem, s>>>(dPb, n, counts, tab, tab64);
+    if (nc == 4) k_solve_batch<4><<<grid, 4 * NGPT, smem, s>>>(dPb, n, counts, tab, tab64);
+    else k_solve_batch<2><<<grid, 2 * NGPT, smem, s>>>(dPb, n, counts, tab, tab64);
     return cudaGetLastError();
 }
 

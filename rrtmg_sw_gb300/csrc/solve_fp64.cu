@@ -1,24 +1,25 @@
-// solve_fp64.cu -- plain FP64 form.  Built with --fmad=false so that every
-// multiply and add rounds separately, as the reference's expressions do;
-// together with the reference's operation order this makes the device
-// results agree with the FP64 oracle to rounding of log/exp only.
-#include "kernel.cuh"
+// solve_fp64.cu -- plain FP64 form.  Built with --fmad=false: a multiply and
+// an add are fused only where the source says fma(), so every kernel that
+// inlines the form's functions gives the same results bit for bit.
+#include "fp64.cuh"
 #include "launch.h"
 
 namespace rrsw {
 
 cudaError_t upload_tables_fp64(const DevTables& t) { return cudaMemcpyToSymbol(cT, &t, sizeof(DevTables)); }
 
-size_t slot_elems(int nlay, int idelm, bool fp32, int nc) {
-    (void)fp32;  // the same level fields in both forms (elements of the form's type)
+size_t slot_elems(int nlay, int idelm, int nc) {
     return (size_t)nlay * (size_t)(idelm == 0 ? NS_MAX : S_DBTCN) * (size_t)(nc * NGPT);
+}
+
+size_t slot_elems_fp64(const SolveParams& P, int nc) {
+    return slot64(P.nlay, P.idelm, nc, band_clouds(P), P.iaer != 0).total;
 }
 
 LaunchInfo plan_fp64(const SolveParams& P, int num_sms) {
     LaunchInfo li;
-    li.smem = smem_layout(P.nlay, num_q<double>(P.extra != 0), stages_clouds(P),
-                          stage_aerosol<double>(P.iaer), sizeof(double)).total;
-    const auto kern = P.mt ? k_solve<double, true> : k_solve<double, false>;
+    li.smem = smem64(P, COLS_PER_CTA).total;
+    const auto kern = P.mt ? k_solve64<true> : k_solve64<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)li.smem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, CTA_THREADS, li.smem);
@@ -26,12 +27,13 @@ LaunchInfo plan_fp64(const SolveParams& P, int num_sms) {
     li.grid = num_sms * per_sm;
     if (li.grid > P.npairs) li.grid = P.npairs;
     if (li.grid < 1) li.grid = 1;
+    li.slot_bytes = slot_elems_fp64(P, COLS_PER_CTA) * sizeof(double);
     return li;
 }
 
 cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s) {
-    if (P.mt) k_solve<double, true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab);
-    else k_solve<double, false><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab);
+    if (P.mt) k_solve64<true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab);
+    else k_solve64<false><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab);
     return cudaGetLastError();
 }
 
@@ -41,13 +43,10 @@ cudaError_t launch_compact(const SolveParams* dPb, int n, int* map_all, const lo
     return cudaGetLastError();
 }
 
-size_t solve_smem_fp64(const SolveParams& P, int nc) {
-    return smem_layout(P.nlay, num_q<double>(P.extra != 0), stages_clouds(P), stage_aerosol<double>(P.iaer),
-                       sizeof(double), nc).total;
-}
+size_t solve_smem_fp64(const SolveParams& P, int nc) { return smem64(P, nc).total; }
 
 int batch_blocks_per_sm_fp64(size_t smem, int nc) {
-    const auto kern = nc == 4 ? k_solve_batch<double, 4> : k_solve_batch<double, 2>;
+    const auto kern = nc == 4 ? k_solve64_batch<4> : k_solve64_batch<2>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nc * NGPT, smem);
@@ -56,8 +55,8 @@ int batch_blocks_per_sm_fp64(size_t smem, int nc) {
 
 cudaError_t launch_batch_fp64(const SolveParams* dPb, int n, const int* counts, const double* tab, int grid,
                               size_t smem, int nc, cudaStream_t s) {
-    if (nc == 4) k_solve_batch<double, 4><<<grid, 4 * NGPT, smem, s>>>(dPb, n, counts, tab, tab);
-    else k_solve_batch<double, 2><<<grid, 2 * NGPT, smem, s>>>(dPb, n, counts, tab, tab);
+    if (nc == 4) k_solve64_batch<4><<<grid, 4 * NGPT, smem, s>>>(dPb, n, counts, tab);
+    else k_solve64_batch<2><<<grid, 2 * NGPT, smem, s>>>(dPb, n, counts, tab);
     return cudaGetLastError();
 }
 
