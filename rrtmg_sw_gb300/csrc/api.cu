@@ -602,6 +602,7 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
     st.last_kernel = !fp32 ? RRTMG_SW_KERNEL_FP64 : li.tiled ? RRTMG_SW_KERNEL_FP32_TILED : RRTMG_SW_KERNEL_FP32;
     st.last_tile_slots = fp32 && li.tiled ? li.tile_slots : 0;
     P.slot_elems = li.slot_bytes / (fp32 ? sizeof(float) : sizeof(double));
+    if (li.split_lb) launches += 1;  // cells, then sweeps
     // tiled: per-CTA areas, then the pairs' prepared blocks, then the overflow list
     const size_t off_prep = ovf_offset((size_t)li.grid * li.slot_bytes);
     const size_t off = ovf_offset(off_prep + (size_t)P.npairs * li.prep_bytes);
@@ -1066,6 +1067,7 @@ int solve_static(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cu
     const size_t doc_bytes = fp32 ? li.slot_bytes : slot_elems(P.nlay, P.idelm) * sizeof(double);
     if (avail / doc_bytes < need) return RRTMG_SW_ESCRATCH;
     const size_t slots = avail / li.slot_bytes;
+    if (li.split_lb && (size_t)li.grid > slots) li = plan_fp64(P, st.num_sms, false);
     if ((size_t)li.grid > slots) li.grid = (int)slots;
     P.slot_elems = li.slot_bytes / (fp32 ? sizeof(float) : sizeof(double));
     StaticArea area;
@@ -1085,7 +1087,7 @@ int solve_static(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cu
     CK(cudaMemsetAsync(P.err, 0, sizeof(int), s));
     if (fp32) CK(launch_solve_fp32(P, (const float*)st.d_tab32.p, (const double*)st.d_tab64.p, li, s));
     else CK(launch_solve_fp64(P, (const double*)st.d_tab64.p, li, s));
-    int launches = li.tiled ? 2 : 1;
+    int launches = li.tiled || li.split_lb ? 2 : 1;
     int h[2] = {0, 0};  // pageable: the copies complete before the calls return
     CK(cudaMemcpyAsync(&h[0], P.err, sizeof(int), cudaMemcpyDeviceToHost, s));
     if (li.tiled) CK(cudaMemcpyAsync(&h[1], P.tovfcount, sizeof(int), cudaMemcpyDeviceToHost, s));

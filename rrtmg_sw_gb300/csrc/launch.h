@@ -19,11 +19,12 @@ struct LaunchInfo {
     int prep_grid = 0;
     size_t prep_smem = 0, prep_bytes = 0;
     int tile_slots = 2;  // pair slots of the tiled kernel (SolveParams::tile_slots)
+    int split_lb = 0;    // FP64 form, few columns: layers per CTA of the split kernels (0: the fused kernel)
 };
 
 // FP64 form
 cudaError_t upload_tables_fp64(const DevTables& t);
-LaunchInfo plan_fp64(const SolveParams& P, int num_sms);
+LaunchInfo plan_fp64(const SolveParams& P, int num_sms, bool allow_split = true);
 cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s);
 // FP32 form
 cudaError_t upload_tables_fp32(const DevTables& t);

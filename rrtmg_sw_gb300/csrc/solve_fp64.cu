@@ -16,8 +16,35 @@ size_t slot_elems_fp64(const SolveParams& P, int nc) {
     return slot64(P.nlay, P.idelm, nc, band_clouds(P), P.iaer != 0).total;
 }
 
-LaunchInfo plan_fp64(const SolveParams& P, int num_sms) {
+// Layers per CTA of the split kernels for a call that takes them, else 0.
+// They are the faster ones wherever they were measured (60 layers, clouds: 1
+// column 0.66 -> 0.17 ms, 63 x 47 1.02 -> 0.29, 304 1.29 -> 0.87, 608 1.81 ->
+// 1.54, 1 024 3.06 -> 2.65, 2 048 5.00 -> 4.55 ms), but they take one scratch slot
+// per column pair, so larger calls keep the fused kernel's one per resident
+// CTA.  The block of layers is the one whose CTAs fill the GPU's rounds of two
+// CTAs per SM best, at one layer's time of preparation per CTA.
+static int split_layers(const SolveParams& P, int num_sms, size_t slot_bytes) {
+    constexpr size_t kMaxScratch = (size_t)2 << 30;
+    if (P.colmap || P.npairs > 8 * num_sms || (size_t)P.npairs * slot_bytes > kMaxScratch) return 0;
+    const long long round = 2ll * num_sms;
+    int best = 1;
+    double cost = 1e30;
+    for (int lb = 1; lb <= SPLIT_MAXLB && lb <= P.nlay; ++lb) {
+        const long long ctas = (long long)P.npairs * ((P.nlay + lb - 1) / lb);
+        const double c = (double)((ctas + round - 1) / round) * (lb + 1.0);
+        if (c < cost) { cost = c; best = lb; }
+    }
+    return best;
+}
+
+LaunchInfo plan_fp64(const SolveParams& P, int num_sms, bool allow_split) {
     LaunchInfo li;
+    li.slot_bytes = slot_elems_fp64(P, COLS_PER_CTA) * sizeof(double);
+    li.split_lb = allow_split ? split_layers(P, num_sms, li.slot_bytes) : 0;
+    if (li.split_lb) {
+        li.grid = P.npairs;  // one slot per pair
+        return li;
+    }
     li.smem = smem64(P, COLS_PER_CTA).total;
     const auto kern = P.mt ? k_solve64<true> : k_solve64<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)li.smem);
@@ -27,11 +54,21 @@ LaunchInfo plan_fp64(const SolveParams& P, int num_sms) {
     li.grid = num_sms * per_sm;
     if (li.grid > P.npairs) li.grid = P.npairs;
     if (li.grid < 1) li.grid = 1;
-    li.slot_bytes = slot_elems_fp64(P, COLS_PER_CTA) * sizeof(double);
     return li;
 }
 
 cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s) {
+    if (li.split_lb) {
+        const size_t sc = split_smem64(P).total, ss = sweep_smem64(P).total;
+        const auto cells = P.mt ? k_cells64<true> : k_cells64<false>;
+        cudaError_t e = cudaFuncSetAttribute(cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sc);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sweep64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ss);
+        if (e != cudaSuccess) return e;
+        const dim3 gc(P.npairs, (P.nlay + li.split_lb - 1) / li.split_lb), gs(P.ncol, cloud_mode(P) == CLD_NONE ? 1 : 2);
+        cells<<<gc, SPLIT_THREADS, sc, s>>>(P, li.split_lb, tab);
+        k_sweep64<<<gs, SWEEP_THREADS, ss, s>>>(P, tab);
+        return cudaGetLastError();
+    }
     if (P.mt) k_solve64<true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab);
     else k_solve64<false><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab);
     return cudaGetLastError();
