@@ -53,8 +53,8 @@ struct State {
     double cpdair = 1.004e3;
     DevBuf d_tab64, d_tab32, scratch, errw, bounds;
     std::map<std::string, DevBuf> stage;  // host-API staging buffers
-    int* h_err = nullptr;                  // pinned: [0] error word, [1] tiled-kernel overflow count
-    unsigned long long* h_stats = nullptr;  // pinned: the FP32 form's counters of the last solve
+    int* h_err = nullptr;                  // pinned: error word (device solves write it directly)
+    unsigned long long* h_stats = nullptr;  // pinned: the FP32 form's counters of the last solve, overflow count
     DevBuf statsw;                         // their device copy
     long long last_stats[4] = {0, 0, 0, 0};
     // from the environment at each rrtmg_sw_ini_c: RRTMG_SW_TILED=0 keeps the
@@ -578,10 +578,12 @@ size_t ovf_bytes(int npairs) { return (size_t)(npairs + 1) * sizeof(int); }
 // Queue one solve on `s` (device pointers in a/c) with the given scratch
 // buffer and device error word; nothing is synchronised.  Pout / liout
 // receive the parameters and launch shape (the tiled FP32 kernel's overflow
-// list is read by the caller).
+// list is read by the caller).  ovf_count: a zeroed device word for the
+// tiled kernel's overflow count (nullptr: one in the scratch, zeroed here).
 int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cudaStream_t s, bool nomcica,
                   DevBuf& scratch, int* err, int& launches, SolveParams* Pout = nullptr,
-                  LaunchInfo* liout = nullptr, bool allow_tiled = true, unsigned long long* stats = nullptr) {
+                  LaunchInfo* liout = nullptr, bool allow_tiled = true, unsigned long long* stats = nullptr,
+                  int* ovf_count = nullptr) {
     SolveParams P;
     int rc = make_params(st, a, c, P, nomcica);
     if (rc) return rc;
@@ -610,12 +612,12 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
     P.scratch = scratch.p;
     if (li.tiled) {
         P.tprep = (char*)scratch.p + off_prep;
-        P.tovfcount = (int*)((char*)scratch.p + off);
-        P.tovf = P.tovfcount + 1;
+        P.tovfcount = ovf_count ? ovf_count : (int*)((char*)scratch.p + off);
+        P.tovf = (int*)((char*)scratch.p + off) + 1;
         P.tovfcap = P.npairs;
         P.tile_qcap = st.tile_qcap;
         P.tile_slots = li.tile_slots;
-        CK(cudaMemsetAsync(P.tovfcount, 0, sizeof(int), s));
+        if (!ovf_count) CK(cudaMemsetAsync(P.tovfcount, 0, sizeof(int), s));
         launches += 1;  // the preparation kernel
     }
     if (fp32) CK(launch_solve_fp32(P, (const float*)st.d_tab32.p, (const double*)st.d_tab64.p, li, s));
@@ -667,41 +669,48 @@ int tiled_fallback(State& st, const SolveParams& Pt, int count, cudaStream_t s, 
     return RRTMG_SW_OK;
 }
 
-// Queue one solve on `s`; returns after reading back the device error word
-// (and, after the tiled FP32 kernel, after solving again any column pairs it
-// could not finish).
+// Queue one solve on `s`; returns with its error word (and, after the tiled
+// FP32 kernel, after solving again any column pairs it could not finish).
+// The kernels write the error word to page-locked host memory themselves;
+// the FP32 form's counters and the tiled kernel's overflow count share one
+// device buffer, zeroed and read back once.  With a memset and a copy for each
+// (and a second synchronisation for the counters), a call of one column spent
+// as long on them as on its kernels.
 int solve_dev(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cudaStream_t s, bool nomcica = false,
               bool allow_tiled = true) {
-    CK(st.errw.ensure(sizeof(int)));
-    int* err = (int*)st.errw.p;
-    CK(cudaMemsetAsync(err, 0, sizeof(int), s));
+    volatile int* err = st.h_err;
+    *err = 0;
     int launches = 0;
     SolveParams P;
     LaunchInfo li;
-    CK(st.statsw.ensure(4 * sizeof(unsigned long long)));
-    CK(cudaMemsetAsync(st.statsw.p, 0, 4 * sizeof(unsigned long long), s));
-    const int rc = enqueue_solve(st, a, c, s, nomcica, st.scratch, err, launches, &P, &li, allow_tiled,
-                                 (unsigned long long*)st.statsw.p);
+    const bool fp32 = st.form == RRTMG_SW_FORM_FP32;
+    unsigned long long* words = nullptr;  // 4 counters, then the overflow count
+    constexpr size_t kWords = 5 * sizeof(unsigned long long);
+    for (int i = 0; i < 5; ++i) st.h_stats[i] = 0;
+    if (fp32) {
+        CK(st.statsw.ensure(kWords));
+        words = (unsigned long long*)st.statsw.p;
+        CK(cudaMemsetAsync(words, 0, kWords, s));
+    }
+    const int rc = enqueue_solve(st, a, c, s, nomcica, st.scratch, st.h_err, launches, &P, &li, allow_tiled, words,
+                                 fp32 ? (int*)(words + 4) : nullptr);
     if (rc) return rc;
-    st.h_err[1] = 0;
-    CK(cudaMemcpyAsync(st.h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    if (li.tiled) CK(cudaMemcpyAsync(st.h_err + 1, P.tovfcount, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (fp32) CK(cudaMemcpyAsync(st.h_stats, words, kWords, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (li.tiled && st.h_err[0] == 0 && st.h_err[1] > 0) {
+    const int ovf = (int)st.h_stats[4];
+    if (li.tiled && *err == 0 && ovf > 0) {
         DevBuf& cm = st.stage["tovf_colmap"];
-        CK(cm.ensure((2 * (size_t)std::min(st.h_err[1], P.tovfcap) + 1) * sizeof(int)));
-        const int r2 = tiled_fallback(st, P, st.h_err[1], s, (int*)cm.p, [&](size_t b) -> void* {
+        CK(cm.ensure((2 * (size_t)std::min(ovf, P.tovfcap) + 1) * sizeof(int)));
+        const int r2 = tiled_fallback(st, P, ovf, s, (int*)cm.p, [&](size_t b) -> void* {
             return st.scratch.ensure(b) == cudaSuccess ? st.scratch.p : nullptr;
         }, launches);
         if (r2) return r2;
-        CK(cudaMemcpyAsync(st.h_err, err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(st.h_stats, words, kWords, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
     }
-    CK(cudaMemcpyAsync(st.h_stats, st.statsw.p, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
     for (int i = 0; i < 4; ++i) st.last_stats[i] = (long long)st.h_stats[i];
     st.last_launches = launches;
-    return bounds_status(st, *st.h_err);
+    return bounds_status(st, *err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1384,8 +1393,8 @@ int rrtmg_sw_ini_c(double cpdair) {
         CK(cudaDeviceGetAttribute(&st.num_sms, cudaDevAttrMultiProcessorCount, dev));
         const int rc = build_tables(st);
         if (rc) return rc;
-        CK(cudaMallocHost((void**)&st.h_err, 2 * sizeof(int)));
-        CK(cudaMallocHost((void**)&st.h_stats, 4 * sizeof(unsigned long long)));
+        CK(cudaMallocHost((void**)&st.h_err, sizeof(int)));
+        CK(cudaMallocHost((void**)&st.h_stats, 5 * sizeof(unsigned long long)));
         CK(cudaStreamCreateWithFlags(&st.host_stream, cudaStreamNonBlocking));
     }
     {
