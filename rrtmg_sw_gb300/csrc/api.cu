@@ -595,9 +595,10 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
         const uint64_t nr = mt_stream_length(P.icld, P.ncol, P.nlay);
         DevBuf& rs = st.stage["mt_stream"];
         CK(rs.ensure((nr + 2) * sizeof(uint32_t)));  // + the mask's read-ahead past the last run
-        CK(launch_mt_jump((uint32_t)P.permuteseed, nr, (uint32_t*)rs.p, st.num_sms, 0, s));
+        int nl = 0;
+        CK(launch_mt_jump((uint32_t)P.permuteseed, nr, (uint32_t*)rs.p, st.num_sms, 0, s, &nl));
         P.mt = (const uint32_t*)rs.p;
-        launches += 2;
+        launches += nl;
     }
     const bool fp32 = st.form == RRTMG_SW_FORM_FP32;
     LaunchInfo li = fp32 ? plan_fp32(P, st.num_sms, allow_tiled && !st.no_tiled) : plan_fp64(P, st.num_sms);
@@ -1508,10 +1509,11 @@ int mcica_subcol_sw_c(int32_t ncol, int32_t nlay, int32_t icld, int32_t permutes
         const uint64_t nr = mt_stream_length(icld, ncol, nlay);
         DevBuf& rs = st.stage["mt_stream"];
         CK(rs.ensure((nr + 2) * sizeof(uint32_t)));  // + the mask's read-ahead past the last run
-        CK(launch_mt_jump((uint32_t)permuteseed, nr, (uint32_t*)rs.p, st.num_sms, 0, s));
+        int nl = 0;
+        CK(launch_mt_jump((uint32_t)permuteseed, nr, (uint32_t*)rs.p, st.num_sms, 0, s, &nl));
         CK(launch_mcica_stream(ncol, nlay, icld, (const uint32_t*)rs.p, d_cf, d_ciwp, d_clwp, d_tauc, d_ssac, d_asmc,
                                d_fsfc, d_alpha, o[0], o[1], o[2], o[3], o[4], o[5], o[6], s));
-        st.last_launches = 3;
+        st.last_launches = nl + 1;
     }
     CK(cudaMemcpyAsync(st.h_err, st.errw.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     for (int i = 0; i < 7; ++i) sg.back(h[i], o[i], G);
@@ -1590,8 +1592,7 @@ int rrtmg_sw_mt_stream_dev_c(int32_t seed, uint64_t n, uint32_t* out, int32_t lo
     std::lock_guard<std::mutex> lk(st.mu);
     if (const int r0 = ready(st)) return r0;
     if (!out || log_seg > 40) return RRTMG_SW_EARGS;
-    CK(launch_mt_jump((uint32_t)seed, n, out, st.num_sms, log_seg, (cudaStream_t)stream));
-    st.last_launches = n ? 2 : 0;
+    CK(launch_mt_jump((uint32_t)seed, n, out, st.num_sms, log_seg, (cudaStream_t)stream, &st.last_launches));
     CK(cudaStreamSynchronize((cudaStream_t)stream));
     return RRTMG_SW_OK;
 }

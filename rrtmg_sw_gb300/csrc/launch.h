@@ -76,7 +76,8 @@ cudaError_t launch_mcica_kiss(int ncol, int nlay, int icld, int permuteseed, con
 // MT19937 stream of the reference generator seeded with seed: n tempered
 // words, segments of 2^log_seg words generated in parallel after a
 // jump-ahead (log_seg <= 0: chosen from n and num_sms) (mt19937.cu)
-cudaError_t launch_mt_jump(uint32_t seed, uint64_t n, uint32_t* out, int num_sms, int log_seg, cudaStream_t s);
+cudaError_t launch_mt_jump(uint32_t seed, uint64_t n, uint32_t* out, int num_sms, int log_seg, cudaStream_t s,
+                           int* launches = nullptr);
 // raw (untempered) words behind outputs offset .. offset+623, on the host;
 // 0 or -1 (offset >= 2^48 or jump tables unavailable)
 int mt_window_host(uint32_t seed, uint64_t offset, uint32_t* window);

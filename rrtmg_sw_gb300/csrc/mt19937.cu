@@ -18,10 +18,12 @@
 // phi is found once on the host by Berlekamp-Massey over 2*19937 output
 // bits (it is primitive, so one bit sequence has it as minimal polynomial);
 // the table x^(2^b) mod phi, b < 48, follows by repeated squaring.  Segment
-// p of length S = 2^s starts at output p*S: one CTA of k_mt_windows composes
-// the jumps of the set bits of p (x^(2^(b+s))) into the segment's first 624
-// words, then one CTA of k_mt_generate (8 per SM) runs the recurrence over
-// the rest of the segment as the sequential generator would.
+// p of length S = 2^s starts at output p*S.  The segments' first 624 words
+// (windows) come from a binary tree of jumps: level b makes segment p + 2^b
+// from segment p by x^(2^(b+s)), so ns segments take ns - 1 jumps in
+// log2(ns) launches of k_mt_jump, each jump's polynomial cut over as many
+// CTAs as leave no SM idle.  Then one CTA of k_mt_generate (8 per SM) runs the
+// recurrence over each segment as the sequential generator would.
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -37,7 +39,6 @@ constexpr int NW = 624, MW = 397, DEG = 19937;
 constexpr int PW = 312;              // 64-bit words of a reduced polynomial (degree < 19937)
 constexpr int EXT = DEG + NW - 1;    // words one jump reads: 20560
 constexpr int MAXB = 48;             // jump table x^(2^b) mod phi, b < MAXB
-constexpr int WTHREADS = 256;        // window kernel: >= 227 (one recurrence step), >= 156 (jump outputs / 4)
 constexpr int GTHREADS = 256;        // generation kernel: >= 227
 constexpr uint64_t RING = 1023;      // generation ring: 1024 words, index mask
 
@@ -273,86 +274,98 @@ cudaError_t device_table(const Tables& T, const uint64_t** out) {
 
 // --------------------------------------------------------------- device side
 
-// In-place regeneration of the 624-word state (three dependency-free
-// phases of 227, 227 and 169 words, then the last word).  Starts with a
-// read phase and a barrier, so the previous block's readers are done
-// before any word is overwritten.
-__device__ inline void regenerate(uint32_t* e, int t) {
-    uint32_t v = 0;
-    if (t < NW - MW) v = e[t + MW] ^ twist(e[t], e[t + 1]);
-    __syncthreads();
-    if (t < NW - MW) e[t] = v;
-    __syncthreads();
-    if (t < NW - MW) v = e[t] ^ twist(e[t + 227], e[t + 228]);
-    __syncthreads();
-    if (t < NW - MW) e[t + 227] = v;
-    __syncthreads();
-    if (t < 169) v = e[t + 227] ^ twist(e[t + 454], e[t + 455]);
-    __syncthreads();
-    if (t < 169) e[t + 454] = v;
-    __syncthreads();
-    if (t == 0) e[NW - 1] = e[MW - 1] ^ twist(e[NW - 1], e[0]);
-    __syncthreads();
+// Window 0 (x_624 .. x_1247, from the host) into the first segment, zeros
+// into the other segments' first 624 words, where k_mt_jump adds up theirs.
+struct Window {
+    uint32_t w[NW];
+};
+__global__ void __launch_bounds__(NW) k_mt_seed(const __grid_constant__ Window w0, uint64_t n, int logS,
+                                                uint32_t* __restrict__ out) {
+    const uint64_t k = ((uint64_t)blockIdx.x << logS) + threadIdx.x;
+    if (k < n) out[k] = blockIdx.x == 0 ? w0.w[threadIdx.x] : 0u;
 }
 
-// Kernel 1: the window of segment p = blockIdx.x (the 624 raw words behind
-// outputs p*2^logS ..), written raw into the first min(624, len) words of
-// the segment's own output range.  Jumps: one per set bit of p; in a jump,
-// thread t < 156 forms output words t, t+156, t+312, t+468 so the bit scan
-// of the polynomial is shared by four accumulators.
-__global__ void __launch_bounds__(WTHREADS) k_mt_windows(uint32_t seed, uint64_t n, int logS,
-                                                        const uint64_t* __restrict__ jump,
-                                                        uint32_t* __restrict__ out) {
-    extern __shared__ __align__(16) uint64_t sm_mt[];
-    uint64_t* sp = sm_mt;                      // jump polynomial, PW words
-    uint32_t* e = (uint32_t*)(sm_mt + PW);     // EXT words
+// One level of the tree: the raw window of segment p + 2^b, p = blockIdx.x,
+// from that of segment p, by the jump polynomial g = x^(2^(b+logS)) mod phi;
+// CTA blockIdx.y adds (XOR) the terms of g's 32-bit words w0 .. w0 + nw.
+//
+// A jump XORs half of 624 x 19937 words; with one shared-memory read for each
+// it is bound by those reads.  Here a thread forms JR = 8 consecutive outputs,
+// so the words it holds serve 8 bits of g each: 39 reads and about 130 XORs
+// per 32 bits and thread, bound by their issue (about 240 000 cycles of an
+// SM).  The words sit in 8 rows by their index mod 8, so that the threads'
+// reads 8 words apart hit consecutive banks.  Measured with the tree: 0.44 M
+// words 0.81 -> 0.10 ms, 4.2 M 2.57 -> 0.17, 110 M 4.94 -> 0.64, 440 M 7.76 -> 1.5 ms.
+constexpr int JR = 8;                    // outputs per thread
+constexpr int JT = NW / JR;              // 78 threads form all outputs
+constexpr int JG = 3;                    // groups of them, each a third of the CTA's words of g (groups of whole
+                                         // warps, 3 x 96 threads: 1.45 times the time)
+constexpr int JTHREADS = 256;            // >= JT * JG, >= 227 (one recurrence step)
+constexpr int JROW = 2596;               // row length: >= (EXT + 39) / 8, 4 mod 32 (conflict-free stores)
+constexpr int GW = 2 * PW;               // 32-bit words of g
+static_assert(JT * JR == NW && JT * JG <= JTHREADS && JROW * JR >= EXT + 40 && JROW % 32 == 4, "jump tile");
+
+__device__ inline int jaddr(int k) { return (k & (JR - 1)) * JROW + (k >> 3); }
+
+__global__ void __launch_bounds__(JTHREADS, 2)
+k_mt_jump(uint64_t n, int logS, int b, int per, const uint32_t* __restrict__ g, uint32_t* __restrict__ out) {
+    extern __shared__ __align__(16) uint32_t sm_jump[];
+    uint32_t* e = sm_jump;               // [JR][JROW]: words after the parent's window
+    uint32_t* sg = sm_jump + JR * JROW;  // this CTA's words of g
     const int t = threadIdx.x;
-    const uint64_t p = blockIdx.x;
-    const uint64_t start = p << logS;
+    const uint64_t p = blockIdx.x, child = p + (1ull << b);
+    const uint64_t start = child << logS;
     if (start >= n) return;
-    if (t == 0) {
-        e[0] = seed;
-        for (int i = 1; i < NW; ++i) e[i] = 1812433253u * (e[i - 1] ^ (e[i - 1] >> 30)) + (uint32_t)i;
+    const int w0 = blockIdx.y * per, w1 = min(GW, w0 + per);
+    int any = 0;
+    for (int w = w0 + t; w < w1; w += JTHREADS) {
+        sg[w - w0] = g[w];
+        any |= g[w] != 0u;
     }
+    if (!__syncthreads_or(any)) return;  // a sparse jump's empty part
+    const uint32_t* win = out + (p << logS);
+    for (int k = t; k < NW; k += JTHREADS) e[jaddr(k)] = win[k];
     __syncthreads();
-    regenerate(e, t);  // x_624..x_1247: outputs 0..623
-    constexpr int Q = NW / 4;
-    for (int b = 0; (p >> b) != 0ull; ++b) {
-        if (!((p >> b) & 1ull)) continue;
-        const uint64_t* g = jump + (size_t)(b + logS) * PW;
-        for (int w = t; w < PW; w += WTHREADS) sp[w] = g[w];
-        // the 19936 + 624 words after the window
-        for (int q = NW; q < EXT; q += NW - MW) {
-            const int k = q + t;
-            if (t < NW - MW && k < EXT) e[k] = e[k - NW + MW] ^ twist(e[k - NW], e[k - NW + 1]);
-            __syncthreads();
-        }
-        uint32_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        if (t < Q) {
-            for (int w = 0; w < PW; ++w) {
-                uint64_t gw = sp[w];
-                const uint32_t* ew = e + 64 * w + t;
-                while (gw) {
-                    const uint32_t* x = ew + (__ffsll((long long)gw) - 1);
-                    gw &= gw - 1;
-                    a0 ^= x[0];
-                    a1 ^= x[Q];
-                    a2 ^= x[2 * Q];
-                    a3 ^= x[3 * Q];
+    // the words up to the last one these bits of g reach
+    const int need = min(EXT, 32 * w1 + NW);
+    for (int q = NW; q < need; q += NW - MW) {
+        const int k = q + t;
+        if (t < NW - MW && k < EXT)
+            e[jaddr(k)] = e[jaddr(k - NW + MW)] ^ twist(e[jaddr(k - NW)], e[jaddr(k - NW + 1)]);
+        __syncthreads();
+    }
+    const int grp = t / JT, j = t % JT;
+    if (grp >= JG) return;
+    const int third = (w1 - w0 + JG - 1) / JG;
+    const int wa = w0 + grp * third, wb = min(w1, wa + third);
+    uint32_t a[JR] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int w = wa; w < wb; ++w) {
+        const uint32_t gw = sg[w - w0];
+        if (!gw) continue;
+        const uint32_t* row = e + (4 * w + j);  // word 32 w + 8 j
+        uint32_t v[2 * JR];
+#pragma unroll
+        for (int c = 0; c < JR; ++c) v[c] = row[c * JROW];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int c = 0; c < JR; ++c) v[JR + c] = row[c * JROW + q + 1];
+#pragma unroll
+            for (int i = 0; i < JR; ++i) {
+                if ((gw >> (JR * q + i)) & 1u) {
+#pragma unroll
+                    for (int r = 0; r < JR; ++r) a[r] ^= v[i + r];
                 }
             }
+#pragma unroll
+            for (int c = 0; c < JR; ++c) v[c] = v[JR + c];
         }
-        __syncthreads();
-        if (t < Q) {
-            e[t] = a0;
-            e[t + Q] = a1;
-            e[t + 2 * Q] = a2;
-            e[t + 3 * Q] = a3;
-        }
-        __syncthreads();
     }
-    const uint64_t len = (n - start) < (1ull << logS) ? (n - start) : (1ull << logS);
-    for (int k = t; k < NW && (uint64_t)k < len; k += WTHREADS) out[start + (uint64_t)k] = e[k];
+#pragma unroll
+    for (int r = 0; r < JR; ++r) {
+        const uint64_t k = start + (uint64_t)(JR * j + r);
+        if (a[r] && k < n) atomicXor(out + k, a[r]);
+    }
 }
 
 // Kernel 2: segment p from its window, 227 words per step through a
@@ -382,14 +395,19 @@ __global__ void __launch_bounds__(GTHREADS) k_mt_generate(uint64_t n, int logS, 
 
 }  // namespace mt
 
-size_t mt_jump_smem() { return mt::PW * sizeof(uint64_t) + (size_t)mt::EXT * sizeof(uint32_t); }
+// CTAs that share a level's jumps: m of them, each cut into parts
+static int jump_parts(uint64_t m, int num_sms) {
+    const uint64_t p = (uint64_t)2 * num_sms / (m ? m : 1);
+    return p < 1 ? 1 : p > 32 ? 32 : (int)p;
+}
 
-// Segment length 2^logS for n words: the windows cost one jump per set
-// bit of the segment index (bits below 2^15 are sparse shifts), the
-// generation one ring step per 227 words; both modelled in SM cycles.
+// Segment length 2^logS for n words, from a model in SM cycles: a level of
+// the tree costs a launch and the words after its windows (12 000), a jump
+// 240 000 cycles of one SM (below 2^15 the polynomial is a power of x: free),
+// the generation one ring step per 227 words.
 static int choose_log_seg(uint64_t n, int num_sms) {
     const double sms = num_sms > 0 ? num_sms : 1;
-    const double jump_cycles = 2.0e5, gen_sm_rate = 3.0, gen_cta_rate = 0.9;  // words per cycle
+    const double level_cycles = 1.2e4, jump_cycles = 2.4e5, gen_sm_rate = 3.0, gen_cta_rate = 0.9;  // words per cycle
     double best = -1.0;
     int pick = 12;
     for (int ls = 12; ls <= 40; ++ls) {
@@ -398,10 +416,12 @@ static int choose_log_seg(uint64_t n, int num_sms) {
         const double resident = per_sm < 8.0 ? per_sm : 8.0;
         const double rate = std::fmin(gen_cta_rate, gen_sm_rate / resident);
         const double waves = std::ceil((double)ns / (8.0 * sms));
-        double dense = 0.0;  // set bits of the segment indices that are dense jumps
-        for (int b = 0; (ns - 1) >> b; ++b)
-            if (b + ls >= 15) dense += (double)ns / 2.0;
-        const double cost = waves * (double)(1ull << ls) / rate + dense * jump_cycles / (2.0 * sms);
+        double cost = waves * (double)(1ull << ls) / rate;
+        for (int b = 0; (ns - 1) >> b; ++b) {
+            const double m = std::fmin((double)(1ull << b), (double)(ns - (1ull << b)));
+            cost += level_cycles;
+            if (b + ls >= 15) cost += std::ceil(m / (2.0 * sms)) * 2.0 * jump_cycles / jump_parts((uint64_t)m, num_sms);
+        }
         if (best < 0.0 || cost < best) {
             best = cost;
             pick = ls;
@@ -411,7 +431,9 @@ static int choose_log_seg(uint64_t n, int num_sms) {
     return pick;
 }
 
-cudaError_t launch_mt_jump(uint32_t seed, uint64_t n, uint32_t* out, int num_sms, int log_seg, cudaStream_t s) {
+cudaError_t launch_mt_jump(uint32_t seed, uint64_t n, uint32_t* out, int num_sms, int log_seg, cudaStream_t s,
+                           int* launches) {
+    if (launches) *launches = 0;
     if (n == 0) return cudaSuccess;
     const mt::Tables& T = mt::tables();
     if (!T.ok) return cudaErrorInvalidValue;
@@ -424,13 +446,23 @@ cudaError_t launch_mt_jump(uint32_t seed, uint64_t n, uint32_t* out, int num_sms
     int top = 0;
     while ((nseg - 1) >> top) ++top;
     if (logS + top > mt::MAXB || nseg > 0x7fffffffull) return cudaErrorInvalidValue;
-    const size_t smem = mt_jump_smem();
-    if ((e = cudaFuncSetAttribute(mt::k_mt_windows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+    const size_t smem = ((size_t)mt::JR * mt::JROW + mt::GW) * sizeof(uint32_t);
+    if ((e = cudaFuncSetAttribute(mt::k_mt_jump, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
         cudaSuccess)
         return e;
-    mt::k_mt_windows<<<(unsigned)nseg, mt::WTHREADS, smem, s>>>(seed, n, logS, dj, out);
+    mt::Window w0;
+    mt::first_window(seed, w0.w);
+    mt::k_mt_seed<<<(unsigned)nseg, mt::NW, 0, s>>>(w0, n, logS, out);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    for (int b = 0; b < top; ++b) {
+        const uint64_t m = nseg - (1ull << b) < (1ull << b) ? nseg - (1ull << b) : (1ull << b);
+        const int parts = jump_parts(m, num_sms), per = (mt::GW + parts - 1) / parts;
+        const uint32_t* g = (const uint32_t*)(dj + (size_t)(b + logS) * mt::PW);
+        mt::k_mt_jump<<<dim3((unsigned)m, (unsigned)parts), mt::JTHREADS, smem, s>>>(n, logS, b, per, g, out);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     mt::k_mt_generate<<<(unsigned)nseg, mt::GTHREADS, 0, s>>>(n, logS, out);
+    if (launches) *launches = 2 + top;
     return cudaGetLastError();
 }
 
