@@ -174,9 +174,9 @@ int rrtmg_sw_nomcica_dev_c(const rrtmg_sw_args *a, const rrtmg_sw_clouds *c, voi
  * Host arrays; c is the fused McICA cloud input (irng = 0) or NULL for
  * clear sky (icld = 0).  rrtmg_sw_ad_c writes J and the gradient arrays
  * (any may be NULL); rrtmg_sw_tl_c reads the same arrays as a direction and
- * writes J and dJ = dJ/dx . direction.  store = 1 keeps each cell's local
- * Jacobian from the forward pass (more memory), 0 recomputes it in the
- * reverse pass, -1 chooses by memory: stored when that scratch fits in half
+ * writes J and dJ = dJ/dx . direction.  store = 1 keeps the
+ * intermediates of each cell's layer solution from the forward pass (more
+ * memory), 0 recomputes them in the reverse pass, -1 chooses by memory: stored when that scratch fits in half
  * of the free device memory; rrtmg_sw_last_ad_store_c reports the choice. */
 typedef struct rrtmg_sw_ad_args {
     double w_toa_up, w_sfc_net, w_hr_sum;
@@ -342,7 +342,7 @@ int rrtmg_sw_last_tile_slots_c(void);
  * second time for their FP64 cells. */
 int rrtmg_sw_last_fp32_stats_c(int64_t* stats);
 /* Checkpointing of the most recent rrtmg_sw_ad_c / rrtmg_sw_tl_c call:
- * 1 stored Jacobians, 0 recomputed, -1 none yet. */
+ * 1 stored intermediates, 0 recomputed, -1 none yet. */
 int rrtmg_sw_last_ad_store_c(void);
 
 /* Reference message for an error code; last CUDA error string. */

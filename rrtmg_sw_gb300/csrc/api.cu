@@ -241,6 +241,12 @@ int build_tables(State& st) {
         if (et[itr] <= expeps) et[itr] = expeps;
     }
     T.exp_tbl = put(et);
+    std::vector<double> e2(2 * 1024);
+    for (int j = 0; j < 1024; ++j) {
+        e2[2 * j] = std::exp2(-j / 1024.0);
+        e2[2 * j + 1] = -std::expm1(-j * (std::log(2.0) / 1024.0));
+    }
+    T.exp2 = put(e2);
     // band/region descriptors of the FP32 gas optics (rrtmg_sw_taumol.f90:275-1785)
     enum { H2O = 0, CO2 = 1, O3 = 2, CH4 = 3, O2 = 4, O2CONT = 9 };
     auto reg = [&](int band, int up, int kind, int sa, int sb, double strrat, double fac, int cont, int minor,
@@ -1184,22 +1190,21 @@ int solve_ad_host(const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, const rrtmg_
     if (P.irng) return RRTMG_SW_EIRNG;
     CK(st.errw.ensure(sizeof(int)));
     P.err = (int*)st.errw.p;
-    const int grid = adjoint_grid(P, st.num_sms);
     if (ad->store < 0) {
-        // stored Jacobians when their scratch fits in half the free memory
+        // stored intermediates when their scratch fits in half the free memory
         // (beyond what is already allocated), else recomputed
         size_t fr = 0, tot = 0;
         CK(cudaMemGetInfo(&fr, &tot));
-        const size_t need = (size_t)grid * adjoint_slot_elems(P.nlay, 1) * sizeof(double);
+        const size_t need = plan_adjoint(P, A.tl, 1, st.num_sms).scratch;
         A.store = need <= st.scratch.bytes + fr / 2 ? 1 : 0;
     }
     st.last_ad_store = A.store;
-    P.slot_elems = adjoint_slot_elems(P.nlay, A.store);
-    CK(st.scratch.ensure((size_t)grid * P.slot_elems * sizeof(double)));
+    const AdPlan plan = plan_adjoint(P, A.tl, A.store, st.num_sms);
+    CK(st.scratch.ensure(plan.scratch));
     P.scratch = st.scratch.p;
     CK(cudaMemsetAsync(P.err, 0, sizeof(int), s));
-    CK(launch_adjoint(P, A, (const double*)st.d_tab64.p, st.num_sms, nullptr, s));
-    st.last_launches = 1;
+    CK(launch_adjoint(P, A, (const double*)st.d_tab64.p, plan, s));
+    st.last_launches = tl ? 2 : 1;
     sg.back(ad->J, A.J, C);
     if (tl) sg.back(ad->dJ, A.dJ, C);
     for (int i = 0; i < 5 && !tl; ++i) sg.back(gh[i], gd[i], CL);

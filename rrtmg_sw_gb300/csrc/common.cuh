@@ -56,6 +56,7 @@ struct DevTables {
     int rsrtaua, rsrpiza, rsrasya;  // (14, 6)
     int wavenum2;
     int exp_tbl;                    // (0:10000)
+    int exp2;                       // 2^(-j/1024) and 1 less it, j = 0 .. 1023, in pairs (adjoint)
     int total;                      // blob size
     int8_t ngb[NGPT];               // band index 0..13 of each g-point
     uint8_t gib[NGPT];              // g index within its band, 1-based

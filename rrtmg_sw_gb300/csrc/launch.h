@@ -50,10 +50,15 @@ cudaError_t launch_batch_fp32(const SolveParams* dPb, int n, const int* counts, 
                               const double* tab64, int grid, size_t smem, int nc, cudaStream_t s);
 // tangent-linear / adjoint (solve_ad.cu)
 cudaError_t upload_tables_ad(const DevTables& t);
-size_t adjoint_slot_elems(int nlay, int store);
-int adjoint_grid(const SolveParams& P, int num_sms);
-cudaError_t launch_adjoint(const SolveParams& P, const AdParams& A, const double* tab64, int num_sms, int* grid_out,
-                           cudaStream_t s);
+struct AdPlan {
+    // k_adjoint and, for the tangent-linear, k_tangent before it: CTAs
+    // (persistent over the column pairs), dynamic shared memory and scratch
+    // doubles per CTA; scratch: bytes of the larger one
+    int grid = 0, tl_grid = 0;
+    size_t smem = 0, tl_smem = 0, slot_elems = 0, tl_slot_elems = 0, scratch = 0;
+};
+AdPlan plan_adjoint(const SolveParams& P, int tl, int store, int num_sms);
+cudaError_t launch_adjoint(SolveParams P, const AdParams& A, const double* tab64, const AdPlan& a, cudaStream_t s);
 // scratch elements per CTA slot of nc columns: of the scratch-based kernels'
 // type (also the size by which rrtmg_sw_static_dev_c refuses a call in either
 // form), and doubles of the FP64 form (fewer than the former)

@@ -70,7 +70,7 @@ struct SolveParams {
 // the device arrays of the objective, its gradients or its direction.
 struct AdParams {
     double w_toa, w_net, w_hr;   // objective weights
-    int store;                   // 1: local Jacobians kept from pass 1, 0: recomputed in the reverse pass
+    int store;                   // 1: layer solutions' intermediates kept from pass 1, 0: recomputed in the reverse pass
     int tl;                      // 1: tangent-linear (dJ along dir), 0: adjoint (gradients)
     double* J;                   // (ncol)
     double* dJ;                  // (ncol), tangent-linear

@@ -350,7 +350,7 @@ def rrtmg_sw_ad(kw, clouds=None, weights=(1.0, 0.0, 0.0), store=True):
     """Adjoint: J and its gradients (dict keyed by AD_LAYER + AD_SFC) for the
     objective J = w_toa_up*swuflx(top) + w_sfc_net*net flux(sfc) + w_hr_sum*sum(swhr);
     ``kw`` holds the rrtmg_sw arguments (as for :func:`rrtmg_sw`).  ``store``:
-    True keeps the local Jacobians, False recomputes them, "auto" lets the
+    True keeps the layer solutions' intermediates, False recomputes them, "auto" lets the
     library choose by free device memory."""
     return _ad_call(kw, clouds, weights, store, None)
 
