@@ -458,19 +458,30 @@ __device__ inline float tbl_exp_beam(float x, const float* __restrict__ tab, flo
 // Layer optics of one cell (rrtmg_sw_spcvmc.f90:442-585): clear optics
 // with aerosol, delta-M scaling, reftra for clear and (if cloudy) total sky,
 // cloud-fraction mixing and the direct beams.  Shared by both forms; the
-// FP32 form also carries the co-albedo and flags risky cells.
-template <typename R>
+// FP32 form also carries the co-albedo and flags risky cells.  AER = false
+// (FP32 form, calls without aerosol): the clear sky's asymmetry is zero, its
+// delta scaling the identity; the statements left out multiply by 0 and by 1.
+// The products and sums whose rounding the compiler's contraction would
+// decide are written out as AER = true has them, so that a call without
+// aerosol and one with aerosol of depth zero agree bit for bit.
+template <typename R, bool AER = true>
 __device__ inline CellOpt<R> cell_optics(const CellIn<R>& ci, int idelm, R prmu0, const R* __restrict__ tab,
                                          const double* __restrict__ tab64, float hrs, float zinc = 0.0f) {
     CellOpt<R> o;
     o.risky = false;
     o.dbtcn = o.dbtn = R(0);
-    R ztauc = ci.taur + ci.taug + ci.rta;
-    R zomcc = ci.taur * R(1) + ci.rta * ci.roa;
-    R zgcc = ci.rga * ci.roa * ci.rta / zomcc;
-    R zcoc = R(0);
-    if constexpr (sizeof(R) == 4) zcoc = (ci.taug + ci.rta * ci.rcoa) / ztauc;  // co-albedo
-    zomcc = zomcc / ztauc;
+    R ztauc, zomcc, zgcc = R(0), zcoc = R(0);
+    if constexpr (AER) {
+        ztauc = ci.taur + ci.taug + ci.rta;
+        zomcc = ci.taur * R(1) + ci.rta * ci.roa;
+        zgcc = ci.rga * ci.roa * ci.rta / zomcc;
+        if constexpr (sizeof(R) == 4) zcoc = (ci.taug + ci.rta * ci.rcoa) / ztauc;  // co-albedo
+        zomcc = zomcc / ztauc;
+    } else {
+        ztauc = __fadd_rn(ci.taur, ci.taug);
+        zcoc = ci.taug / ztauc;
+        zomcc = ci.taur / ztauc;
+    }
     const R zclear = R(1) - ci.cldf, zcloud = ci.cldf;
     if (idelm == 0) {
         const R zdbtmc = tbl_exp<R>(ztauc / prmu0, tab);
@@ -479,14 +490,18 @@ __device__ inline CellOpt<R> cell_optics(const CellIn<R>& ci, int idelm, R prmu0
         o.dbtcn = zdbtmc;
         o.dbtn = zclear * zdbtmc + zcloud * zdbtmo;
     }
-    // delta scaling, clear (spcvmc:492-496)
-    const R zf = zgcc * zgcc;
-    const R zwf = zomcc * zf;
-    ztauc = (R(1) - zwf) * ztauc;
-    zomcc = (zomcc - zwf) / (R(1) - zwf);
-    zgcc = (zgcc - zf) / (R(1) - zf);
-    if constexpr (sizeof(R) == 4) zcoc = zcoc / (R(1) - zwf);
-    o.rc = reftra_g<R>(ztauc, zomcc, zcoc, zgcc, prmu0, tab, tab64);
+    if constexpr (AER) {
+        // delta scaling, clear (spcvmc:492-496)
+        const R zf = zgcc * zgcc;
+        const R zwf = zomcc * zf;
+        ztauc = (R(1) - zwf) * ztauc;
+        zomcc = (zomcc - zwf) / (R(1) - zwf);
+        zgcc = (zgcc - zf) / (R(1) - zf);
+        if constexpr (sizeof(R) == 4) zcoc = zcoc / (R(1) - zwf);
+        o.rc = reftra_g<R>(ztauc, zomcc, zcoc, zgcc, prmu0, tab, tab64);
+    } else {
+        o.rc = reftra_f32_g0(ztauc, zomcc, zcoc, prmu0, tab);
+    }
     const R xc = ztauc / prmu0;
     if constexpr (sizeof(R) == 4) {
         bool br = false;
@@ -501,10 +516,17 @@ __device__ inline CellOpt<R> cell_optics(const CellIn<R>& ci, int idelm, R prmu0
         // total sky: clear + delta-scaled cloud (spcvmc:500-505); reftra
         // only where cldf > repclc (:427); mixed by cloud fraction (:546-549)
         const R ztauo = ztauc + ci.tc;
-        R zomco = ztauc * zomcc + ci.tc * ci.oc;
-        const R zgco = (ci.tc * ci.oc * ci.gc + ztauc * zomcc * zgcc) / zomco;
-        R zcoo = R(0);
-        if constexpr (sizeof(R) == 4) zcoo = (ztauc * zcoc + ci.tc * ci.coc) / ztauo;
+        R zomco, zgco, zcoo = R(0);
+        if constexpr (AER) {
+            zomco = ztauc * zomcc + ci.tc * ci.oc;
+            zgco = (ci.tc * ci.oc * ci.gc + ztauc * zomcc * zgcc) / zomco;
+            if constexpr (sizeof(R) == 4) zcoo = (ztauc * zcoc + ci.tc * ci.coc) / ztauo;
+        } else {
+            const float to = __fmul_rn(ci.tc, ci.oc);
+            zomco = __fadd_rn(__fmul_rn(ztauc, zomcc), to);
+            zgco = to * ci.gc / zomco;
+            zcoo = fmaf(ztauc, zcoc, __fmul_rn(ci.tc, ci.coc)) / ztauo;
+        }
         zomco = zomco / ztauo;
         RT<R> ro;
         if (ci.cldf > R(1.e-12)) {

@@ -72,21 +72,32 @@ __device__ inline bool entry_edge(float x, float eps) {
     return fminf(fr, 1.0f - fr) < 10000.0f * b * x / (bx * bx) * eps;
 }
 
-template <>
-__device__ __forceinline__ RT<float> reftra_g<float>(float zto1, float zw, float zco, float zg, float prmuz,
-                                           const float* __restrict__ tab, const double* __restrict__ tab64,
-                                           int force) {
+// G0: the asymmetry zg is zero (gamma3 = gamma4 = 1/2, za1 = za2, q = 0 in the
+// conservative test); same results bit for bit with a third fewer operations
+// (gamma1's product rounded before the subtraction, as the general form has it).
+template <bool G0>
+__device__ __forceinline__ RT<float> reftra_f32(float zto1, float zw, float zco, float zg, float prmuz,
+                                                const float* __restrict__ tab, int force) {
     RT<float> o;
     const float eps = 1.e-08f;
-    const float zg3 = 3.0f * zg;
-    const float zgamma1 = (8.0f - zw * (5.0f + zg3)) * 0.25f;
-    const float zgamma2 = 3.0f * (zw * (1.0f - zg)) * 0.25f;
-    const float zgamma3 = (2.0f - zg3 * prmuz) * 0.25f;
-    const float zgamma4 = 1.0f - zgamma3;
+    const float zg3 = G0 ? 0.0f : 3.0f * zg;
+    const float zgamma1 = G0 ? __fadd_rn(8.0f, -__fmul_rn(zw, 5.0f)) * 0.25f : (8.0f - zw * (5.0f + zg3)) * 0.25f;
+    const float zgamma2 = G0 ? 3.0f * zw * 0.25f : 3.0f * (zw * (1.0f - zg)) * 0.25f;
+    const float zgamma3 = G0 ? 0.5f : (2.0f - zg3 * prmuz) * 0.25f;
+    const float zgamma4 = G0 ? 0.5f : 1.0f - zgamma3;
     // zwo >= zwcrit  <=>  1 - zwo <= 5e-7  (reftra:183-188)
-    (void)tab64;
     bool edge;
-    const bool cons = conservative_test(zw, zco, zg, edge) <= 5.0e-7f;
+    bool cons;
+    if constexpr (G0) {
+        // conservative_test with q = 0: 1 - zwo = zco
+        const float r = zw > 0.0f ? zco : 1.0f;
+        const float dist = fabsf(r - 5.0e-7f);
+        edge = zw > 0.0f && !(dist > 0.0631f * fabsf(zco) + 1.0e-12f) &&
+               dist <= __fadd_rn(__fmul_rn(2.0e-6f, zco), 1.0e-13f);
+        cons = r <= 5.0e-7f;
+    } else {
+        cons = conservative_test(zw, zco, zg, edge) <= 5.0e-7f;
+    }
     o.adir = 0.0f;
     o.adif = 0.0f;
     o.risky = edge;
@@ -105,8 +116,8 @@ __device__ __forceinline__ RT<float> reftra_g<float>(float zto1, float zw, float
         if (ze2 == 1.0f) { o.ref = 0.0f; o.tra = 1.0f; o.refd = 0.0f; o.trad = 1.0f; }
         return o;
     }
-    const float za1 = zgamma1 * zgamma4 + zgamma2 * zgamma3;
-    const float za2 = zgamma1 * zgamma3 + zgamma2 * zgamma4;
+    const float za1 = G0 ? 0.5f * (zgamma1 + zgamma2) : zgamma1 * zgamma4 + zgamma2 * zgamma3;
+    const float za2 = G0 ? za1 : zgamma1 * zgamma3 + zgamma2 * zgamma4;
     const float zrk = sqrtf(2.0f * zco * (zgamma1 + zgamma2));
     const float zrp = zrk * prmuz;
     const float zrp1 = 1.0f + zrp, zrm1 = 1.0f - zrp;
@@ -155,6 +166,19 @@ __device__ __forceinline__ RT<float> reftra_g<float>(float zto1, float zw, float
     return o;
 }
 
+template <>
+__device__ __forceinline__ RT<float> reftra_g<float>(float zto1, float zw, float zco, float zg, float prmuz,
+                                           const float* __restrict__ tab, const double* __restrict__ tab64,
+                                           int force) {
+    (void)tab64;
+    return reftra_f32<false>(zto1, zw, zco, zg, prmuz, tab, force);
+}
+
+__device__ __forceinline__ RT<float> reftra_f32_g0(float zto1, float zw, float zco, float prmuz,
+                                                   const float* __restrict__ tab) {
+    return reftra_f32<true>(zto1, zw, zco, 0.0f, prmuz, tab, -1);
+}
+
 __device__ __noinline__ RT<float> reftra_f32_cloudy(float zto1, float zw, float zco, float zg, float prmuz,
                                                     const float* __restrict__ tab,
                                                     const double* __restrict__ tab64) {
@@ -183,6 +207,11 @@ cudaError_t launch_setcoef_f32(const SolveParams& P, const float* tab, const dou
 
 cudaError_t upload_tables_fp32(const DevTables& t) { return cudaMemcpyToSymbol(cT, &t, sizeof(DevTables)); }
 
+// The tiled kernel's instance for a call: without aerosol a clear cell's
+// optics need a third fewer operations (262 144 x 60 with McICA clouds
+// 105.7 -> 97.0 ms, 1024 x 60 clear 512 -> 495 us).
+static auto tiled_kernel(const SolveParams& P) { return P.iaer != 0 ? k_solve_tiled<true> : k_solve_tiled<false>; }
+
 LaunchInfo plan_fp32(const SolveParams& P, int num_sms, bool allow_tiled) {
     LaunchInfo li;
     static int smem_optin = -1;
@@ -197,7 +226,7 @@ LaunchInfo plan_fp32(const SolveParams& P, int num_sms, bool allow_tiled) {
         li.tiled = true;
         li.tile_slots = tiled_slots(P, (size_t)smem_optin);
         li.smem = tiled_smem(P.nlay, P.extra ? 16 : 8, fused, fused || nomc, li.tile_slots).total;
-        cudaFuncSetAttribute(k_solve_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)li.smem);
+        cudaFuncSetAttribute(tiled_kernel(P), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)li.smem);
         li.grid = num_sms < P.npairs ? num_sms : P.npairs;
         if (li.grid < 1) li.grid = 1;
         li.slot_bytes = tiled_glob(P.nlay).total;
@@ -231,7 +260,7 @@ cudaError_t launch_solve_fp32(const SolveParams& P, const float* tab, const doub
     if (li.tiled) {
         if (P.mt) k_tiled_prep<true><<<li.prep_grid, CTA_THREADS, li.prep_smem, s>>>(P, tab, tab64);
         else k_tiled_prep<false><<<li.prep_grid, CTA_THREADS, li.prep_smem, s>>>(P, tab, tab64);
-        k_solve_tiled<<<li.grid, T_THREADS, li.smem, s>>>(P, tab, tab64);
+        tiled_kernel(P)<<<li.grid, T_THREADS, li.smem, s>>>(P, tab, tab64);
     } else {
         if (P.mt) k_solve<true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab64);
         else k_solve<false><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab, tab64);

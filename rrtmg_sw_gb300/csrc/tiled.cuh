@@ -570,6 +570,7 @@ __device__ void tiled_load(const SolveParams& P, const TCtx& X, int lp) {
 }
 
 // ---- optics warps: the cells of tile t of pair lp into buffer b
+template <bool AER>
 __device__ void tiled_optics(const SolveParams& P, const TCtx& X, int lp, int t, int b,
                              const float* __restrict__ tab, const double* __restrict__ tab64) {
     const TileView& V = X.V;
@@ -598,19 +599,17 @@ __device__ void tiled_optics(const SolveParams& P, const TCtx& X, int lp, int t,
             CellIn<float> ci;
             ci.taug = taug;
             ci.taur = taur;
-            if (P.iaer != 0) {
+            if constexpr (AER) {
                 ci.rta = aer[(0 * NBND + ib) * L + r];
                 ci.rcoa = aer[(1 * NBND + ib) * L + r];
                 ci.roa = 1.0f - ci.rcoa;
                 ci.rga = aer[(2 * NBND + ib) * L + r];
-            } else {
-                ci.rta = 0.0f; ci.roa = 1.0f; ci.rga = 0.0f; ci.rcoa = 0.0f;
             }
             bool cloudy = false;
             if (X.fused) cloudy = (V.mask[s * 2 + (r >> 5)] >> (r & 31)) & 1u;
             cloud_in<float>(P, pcol, g, lay, ib, X.fused, cloudy, cld, ci, tab);
             const float hrs = zinc * V.hrf[c2 * L + r];
-            const CellOpt<float> co = cell_optics<float>(ci, 1, mu, tab, tab64, hrs, zinc);
+            const CellOpt<float> co = cell_optics<float, AER>(ci, 1, mu, tab, tab64, hrs, zinc);
             f[TF_REFC] = co.rc.ref; f[TF_REFDC] = co.rc.refd; f[TF_ADIRC] = co.rc.adir; f[TF_ADIFC] = co.rc.adif;
             f[TF_DBTC] = co.zdbtc;
             f[TF_REF] = co.rt.ref; f[TF_REFD] = co.rt.refd; f[TF_ADIR] = co.rt.adir; f[TF_ADIF] = co.rt.adif;
@@ -1083,6 +1082,8 @@ __device__ void tiled_zero_bands(const SolveParams& P, const TCtx& X, int lp) {
     __syncwarp();
 }
 
+// AER: the call has aerosol (P.iaer != 0)
+template <bool AER>
 __global__ void __launch_bounds__(T_THREADS, 1)
 k_solve_tiled(const SolveParams P, const float* __restrict__ tab, const double* __restrict__ tab64) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1150,7 +1151,7 @@ k_solve_tiled(const SolveParams P, const float* __restrict__ tab, const double* 
             for (int t = 0; t < TILES; ++t) {
                 const int T = TILES * lp + t, b = T & 1;
                 if (T >= 2) mbar_wait(&X.V.bar[TB_EMPTY0 + b], ((T - 2) >> 1) & 1, X.abort, P.err);
-                tiled_optics(P, X, lp, t, b, tab, tab64);
+                tiled_optics<AER>(P, X, lp, t, b, tab, tab64);
                 opt_sync();  // the tile's cells and risky bits are all written
                 tiled_set_aside(X, lp, t, b);
                 __syncwarp();
