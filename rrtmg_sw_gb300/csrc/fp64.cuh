@@ -390,21 +390,7 @@ __host__ __device__ inline SplitSmem64 split_smem64(const SolveParams& P) {
 // shift register by the matrices of n's bits (the fused kernel's per-launch
 // matrix costs more than one pair saves).
 __device__ inline Kiss kiss_at(const uint32_t* seed, uint64_t n) {
-    const KissJump J = kiss_jump_consts(n);
-    Kiss k;
-    k.s1 = J.A * seed[0] + J.C;
-    uint32_t y = seed[1];
-    for (int b = 0; b < 32 && (n >> b); ++b) {
-        if (!((n >> b) & 1)) continue;
-        uint32_t r = 0;
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) r ^= (0u - (y >> i & 1u)) & cT.xs_jump[b][i];
-        y = r;
-    }
-    k.s2 = y;
-    k.s3 = (uint32_t)mulmod(J.a3n, seed[2], KISS_M3);
-    k.s4 = (uint32_t)mulmod(J.a4n, seed[3], KISS_M4);
-    return k;
+    return kiss_start(seed, kiss_jump_consts(n), xorshift_at(n, seed[1]));
 }
 
 // Layers lay0 + 1 .. lay0 + lb of pair blockIdx.x, lay0 = blockIdx.y lb: the

@@ -809,8 +809,7 @@ __device__ inline KissJump kiss_setup(const SolveParams& P, uint32_t* sXs, int g
     KissJump J{1u, 0u, 1u, 1u};
     if (P.fused && P.icld >= 1) {
         J = kiss_jump_consts(kiss_offset(P.icld, g, P.nlay, P.permuteseed));
-        if (threadIdx.x < NGPT)
-            xorshift_power(kiss_offset(P.icld, threadIdx.x, P.nlay, P.permuteseed), sXs + threadIdx.x * 32);
+        xorshift_matrices(P.icld, P.nlay, P.permuteseed, sXs);
     }
     return J;
 }

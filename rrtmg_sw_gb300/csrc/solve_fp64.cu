@@ -170,8 +170,6 @@ __global__ void k_mcica_kiss(int ncol, int nlay, int icld, int permuteseed, cons
     const int g = (int)(t % NGPT), col = (int)(t / NGPT);
     const size_t n = (size_t)ncol;
     const uint64_t off = kiss_offset(icld, g, nlay, permuteseed);
-    uint32_t xcol[32];
-    xorshift_power(off, xcol);
     uint32_t seed[4];
     const double p1 = __dmul_rn(play[col], 1.e2), p2 = __dmul_rn(play[col + n], 1.e2);
     if (p1 < p2) set_error(err, E_KISSSEED);
@@ -180,7 +178,7 @@ __global__ void k_mcica_kiss(int ncol, int nlay, int icld, int permuteseed, cons
     seed[2] = kiss_seed(__dmul_rn(play[col + 2 * n], 1.e2));
     seed[3] = kiss_seed(__dmul_rn(play[col + 3 * n], 1.e2));
     McicaMask<false> mc;
-    mc.start(kiss_start(seed, kiss_jump_consts(off), xcol), icld);
+    mc.start(kiss_start(seed, kiss_jump_consts(off), xorshift_at(off, seed[1])), icld);
     for (int lay = 1; lay <= nlay; ++lay) {
         const size_t kl = (size_t)col + n * (size_t)(lay - 1);
         double cf = cldfrac[kl];

@@ -408,8 +408,13 @@ k_tiled_prep(const SolveParams P, const float* __restrict__ tab, const double* _
         d.pad = 0;
         tm[i] = d;
     }
-    // KISS: the xorshift part of each subcolumn's stream jump (depends on g)
-    if (fused && !MT && tid < NGPT) xorshift_power(kiss_offset(P.icld, tid, L, P.permuteseed), xs + tid * 32);
+    // KISS: the xorshift part of each subcolumn's stream jump (depends on g),
+    // as a matrix where a CTA takes many pairs.  The matrices cost about 25 us
+    // per launch, a jump without them a few us per pair of a CTA: 64 x 60
+    // columns 301 us without, 324 with them; the line may lie anywhere from 4
+    // to 64 pairs per CTA (4096 to 40 000 columns: within 1 %).
+    const bool jump_matrix = P.npairs > 16 * (int)gridDim.x;
+    if (fused && !MT && jump_matrix) xorshift_matrices(P.icld, L, P.permuteseed, xs);
     const int s = tid, c2s = s / NGPT, g = s % NGPT;
     const int ib = cT.ngb[g], igb = cT.gib[g];
     KissJump J{1u, 0u, 1u, 1u};
@@ -516,7 +521,11 @@ k_tiled_prep(const SolveParams P, const float* __restrict__ tab, const double* _
                 if (act) {
                     McicaMask<MT> mc;
                     Kiss k0{1u, 1u, 1u, 1u};
-                    if constexpr (!MT) k0 = kiss_start(sseed + c2 * 4, J, xs + g * 32);
+                    if constexpr (!MT) {
+                        const uint32_t* sd = sseed + c2 * 4;
+                        k0 = jump_matrix ? kiss_start(sd, J, xs + g * 32)
+                                         : kiss_start(sd, J, xorshift_at(kiss_offset(P.icld, g, L, P.permuteseed), sd[1]));
+                    }
                     mc.start(k0, P.icld, MT ? P.mt + mt_offset(P.icld, g, pcol, P.ncol, L) : nullptr);
                     for (int lay = 1; lay <= L; ++lay) {
                         const int i = lay - 1;
