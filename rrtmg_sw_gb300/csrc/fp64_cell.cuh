@@ -26,10 +26,11 @@
 //     the diffuse flux below a layer follows from the fluxes above it through
 //     the division that the up-sweep has done already.
 //
-// About 170 FP64 instructions per cell (with aerosol) where the reference's
-// order of operations took about 570: 16 384 x 60 columns with clouds and
-// aerosol 102.9 -> 37.6 ms, 1 024 x 60 clear 7.04 -> 2.34 ms, the FP64 pipe 84 %
-// busy.  The layer solution is also written without the cancellation of
+// About 168 FP64 instructions per cell (with aerosol; without, a dozen fewer
+// in the layer solution alone: gamma3 = gamma4 = 1/2 and one alpha) where the
+// reference's order of operations took about 570: 16 384 x 60 columns with
+// clouds and aerosol 102.9 -> 36.8 ms, 4 096 x 60 with clouds 28.2 -> 8.4 ms,
+// the FP64 pipe 84 % busy.  The layer solution is also written without the cancellation of
 // thin layers: against a solve in 80-bit arithmetic the heating rates of
 // 1 024 x 60 clear columns are 8.6e-11 off (2-norm), 1.04e-10 in the
 // reference's order.  Cells near the two-stream resonance k mu0 = 1, where the
@@ -313,33 +314,41 @@ __device__ __forceinline__ Rt64 two_stream64(double tau, double s, double sg, do
         if (__double_as_longlong(e2) == __double_as_longlong(1.0)) { o.ref = 0.0; o.refd = 0.0; o.trad = 1.0; o.tdif = 0.0; }
         return o;
     }
-    const double sum = fma(-0.5, w, fma(-1.5, wg, 2.0));  // gamma1 + gamma2
-    const double g1 = fma(0.5, sum, co);
-    const double g2 = fma(0.5, sum, -co);
-    const double co2 = co + co;
-    const double k = sqrt64(co2 * sum);
-    const double a1 = fma(g2, g3, g1 * g4);
-    const double a2 = fma(g1, g3, g2 * g4);
+    const double h = fma(-0.25, w, G ? fma(-0.75, wg, 1.0) : 1.0);  // (gamma1 + gamma2) / 2
+    const double g1 = h + co, g2 = h - co;
+    const double k = sqrt64(4.0 * co * h);
     const double kmu = k * m.mu;
     const double p1 = 1.0 + kmu, m1 = 1.0 - kmu;
     const double pp = p1 * m1;  // 1 - (k mu0)^2
     double om1;
     const double e1 = tbl_exp64(clip500(k * tau), tab, om1);
-    const double ee = e1 * e1, oo = om1 * (1.0 + e1);  // exp(-2 k tau) and 1 less it
-    const double B = fma(g1, oo, fma(k, ee, k));
+    const double oo = om1 * (1.0 + e1), k2 = k + k;  // oo = 1 - exp(-2 k tau)
+    const double B = fma(g1 - k, oo, k2);
     const double pB = pp * B;  // zdenr zem1
     // (or |zdenr| <= 1e-8, where the reference replaces the solution)
-    if (lt_pos(fabs(pp), RESONANCE64 * w) || lt_pos(fabs(pB), 1.1e-8)) near = true;
+    if (fabsf(to32(pp)) < (float)RESONANCE64 * to32(w) || lt_pos(fabs(pB), 1.1e-8)) near = true;
     const double r = rcp64(pB);
     const double rB = r * pp;        // 1 / B
-    const double k2 = k + k;
-    const double r2 = p1 * fma(-k, g3, a2), r3 = k2 * fma(-a2, m.mu, g3);
-    const double t2 = m1 * fma(-k, g4, a1), t3 = k2 * fma(a1, m.mu, g4);
     const double wr = w * r;
     // zr1 - zr2 ee - zr3 e1 e2 and zt3 e1 - e2 (zt1 - zt2 ee) with
-    // zr1 = zr2 + zr3 and zt1 = zt2 + zt3: no cancellation in thin layers
-    o.ref = wr * fma(r2, oo, r3 * fma(e1, om2, om1));
-    o.tdif = wr * fma(t3, om2 - om1, -e2 * (t2 * oo));
+    // zr1 = zr2 + zr3 and zt1 = zt2 + zt3: no cancellation in thin layers.
+    // Without asymmetry gamma3 = gamma4 = 1/2, alpha1 = alpha2 = h.
+    double r3, t3, r2o, t2o;  // zr3, zt3, zr2 oo, zt2 oo
+    if constexpr (G) {
+        const double a1 = fma(g2, g3, g1 * g4), a2 = fma(g1, g3, g2 * g4);
+        r3 = fma(-a2, m.mu, g3);
+        t3 = fma(a1, m.mu, g4);
+        r2o = p1 * fma(-k, g3, a2) * oo;
+        t2o = m1 * fma(-k, g4, a1) * oo;
+    } else {
+        const double q = fma(-0.5, k, h) * oo;
+        r3 = fma(-h, m.mu, 0.5);
+        t3 = fma(h, m.mu, 0.5);
+        r2o = p1 * q;
+        t2o = m1 * q;
+    }
+    o.ref = wr * fma(k2 * r3, fma(e1, om2, om1), r2o);
+    o.tdif = wr * fma(k2 * t3, om2 - om1, -e2 * t2o);
     o.refd = g2 * oo * rB;
     o.trad = k2 * e1 * rB;
     return o;
