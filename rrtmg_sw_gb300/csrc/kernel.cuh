@@ -285,7 +285,7 @@ __device__ inline float conservative_test(float zw, float zco, float zg, bool& e
     edge = false;
     if (zg == 1.0f) return zw > 0.0f ? zco : 1.0f;
     if (!(zw > 0.0f)) return 1.0f;
-    const float q = zg / (1.0f - zg);
+    const float q = quot(zg, 1.0f - zg);
     const float q2 = q * q;
     const float den = 1.0f - zco * q2;
     if (den == 0.0f) {
@@ -442,7 +442,7 @@ constexpr float BEAM_F_TOL = 1.0e-3f;
 // one entry's step in exp(-x) is e (b + x)^2 / (1e4 b).
 __device__ inline float tbl_exp_beam(float x, const float* __restrict__ tab, float hrs, float zinc, bool& risky) {
     if (x <= 0.06f) return 1.0f - x + 0.5f * x * x;
-    const float u = x / (cT.bpade_f + x);
+    const float u = quot(x, cT.bpade_f + x);
     const float t = 10000.0f * u + 0.5f;
     const int itind = (int)t;
     const float e = ldt(tab, cT.exp_tbl + itind);
@@ -474,13 +474,13 @@ __device__ inline CellOpt<R> cell_optics(const CellIn<R>& ci, int idelm, R prmu0
     if constexpr (AER) {
         ztauc = ci.taur + ci.taug + ci.rta;
         zomcc = ci.taur * R(1) + ci.rta * ci.roa;
-        zgcc = ci.rga * ci.roa * ci.rta / zomcc;
-        if constexpr (sizeof(R) == 4) zcoc = (ci.taug + ci.rta * ci.rcoa) / ztauc;  // co-albedo
-        zomcc = zomcc / ztauc;
+        zgcc = quot(ci.rga * ci.roa * ci.rta, zomcc);
+        if constexpr (sizeof(R) == 4) zcoc = quot(ci.taug + ci.rta * ci.rcoa, ztauc);  // co-albedo
+        zomcc = quot(zomcc, ztauc);
     } else {
         ztauc = __fadd_rn(ci.taur, ci.taug);
-        zcoc = ci.taug / ztauc;
-        zomcc = ci.taur / ztauc;
+        zcoc = quot(ci.taug, ztauc);
+        zomcc = quot(ci.taur, ztauc);
     }
     const R zclear = R(1) - ci.cldf, zcloud = ci.cldf;
     if (idelm == 0) {
@@ -495,14 +495,14 @@ __device__ inline CellOpt<R> cell_optics(const CellIn<R>& ci, int idelm, R prmu0
         const R zf = zgcc * zgcc;
         const R zwf = zomcc * zf;
         ztauc = (R(1) - zwf) * ztauc;
-        zomcc = (zomcc - zwf) / (R(1) - zwf);
-        zgcc = (zgcc - zf) / (R(1) - zf);
-        if constexpr (sizeof(R) == 4) zcoc = zcoc / (R(1) - zwf);
+        zomcc = quot(zomcc - zwf, R(1) - zwf);
+        zgcc = quot(zgcc - zf, R(1) - zf);
+        if constexpr (sizeof(R) == 4) zcoc = quot(zcoc, R(1) - zwf);
         o.rc = reftra_g<R>(ztauc, zomcc, zcoc, zgcc, prmu0, tab, tab64);
     } else {
         o.rc = reftra_f32_g0(ztauc, zomcc, zcoc, prmu0, tab);
     }
-    const R xc = ztauc / prmu0;
+    const R xc = quot(ztauc, prmu0);
     if constexpr (sizeof(R) == 4) {
         bool br = false;
         o.zdbtc = tbl_exp_beam(xc, tab, hrs, zinc, br);
@@ -519,15 +519,15 @@ __device__ inline CellOpt<R> cell_optics(const CellIn<R>& ci, int idelm, R prmu0
         R zomco, zgco, zcoo = R(0);
         if constexpr (AER) {
             zomco = ztauc * zomcc + ci.tc * ci.oc;
-            zgco = (ci.tc * ci.oc * ci.gc + ztauc * zomcc * zgcc) / zomco;
-            if constexpr (sizeof(R) == 4) zcoo = (ztauc * zcoc + ci.tc * ci.coc) / ztauo;
+            zgco = quot(ci.tc * ci.oc * ci.gc + ztauc * zomcc * zgcc, zomco);
+            if constexpr (sizeof(R) == 4) zcoo = quot(ztauc * zcoc + ci.tc * ci.coc, ztauo);
         } else {
             const float to = __fmul_rn(ci.tc, ci.oc);
             zomco = __fadd_rn(__fmul_rn(ztauc, zomcc), to);
-            zgco = to * ci.gc / zomco;
-            zcoo = fmaf(ztauc, zcoc, __fmul_rn(ci.tc, ci.coc)) / ztauo;
+            zgco = quot(to * ci.gc, zomco);
+            zcoo = quot(fmaf(ztauc, zcoc, __fmul_rn(ci.tc, ci.coc)), ztauo);
         }
-        zomco = zomco / ztauo;
+        zomco = quot(zomco, ztauo);
         RT<R> ro;
         if (ci.cldf > R(1.e-12)) {
             if constexpr (sizeof(R) == 4) ro = reftra_f32_cloudy(ztauo, zomco, zcoo, zgco, prmu0, tab, tab64);

@@ -13,7 +13,7 @@ __device__ inline float tbl_exp_om(float x, const float* __restrict__ tab, float
         om = x * (1.0f - 0.5f * x);
         return 1.0f - om;
     }
-    const float tblind = x / (cT.bpade_f + x);
+    const float tblind = quot(x, cT.bpade_f + x);
     const int itind = (int)(10000.0f * tblind + 0.5f);
     const float e = ldt(tab, cT.exp_tbl + itind);
     om = 1.0f - e;
@@ -107,7 +107,7 @@ __device__ __forceinline__ RT<float> reftra_f32(float zto1, float zw, float zco,
         const float za1 = zgamma1 * prmuz - zgamma3;
         const float zgt = zgamma1 * zto1;
         float om;
-        const float ze2 = tbl_exp_om(fminf(zto1 / prmuz, 500.0f), tab, om);
+        const float ze2 = tbl_exp_om(fminf(quot(zto1, prmuz), 500.0f), tab, om);
         const float r1 = 1.0f / (1.0f + zgt);
         o.ref = (zgt - za1 * om) * r1;
         o.tra = (1.0f + za1 * om) * r1;
@@ -136,15 +136,15 @@ __device__ __forceinline__ RT<float> reftra_f32(float zto1, float zw, float zco,
     const float zbeta = g2k * r_kg;
     float om1, om2;
     const float zem1 = tbl_exp_om(fminf(zrk * zto1, 500.0f), tab, om1);
-    const float zem2 = tbl_exp_om(fminf(zto1 / prmuz, 500.0f), tab, om2);
+    const float zem2 = tbl_exp_om(fminf(quot(zto1, prmuz), 500.0f), tab, om2);
     // force = 1 (cloudy total sky): a neighbouring table entry moves pref/ptra
     // of a thick layer enough to show in the fluxes, so every lookup is tested
     if ((force == 1 || fabsf(zrpp) < RESONANCE_WIDE) && !o.risky) {
         const float eps = fabsf(zrpp) < RESONANCE_WIDE ? RESONANCE_EPS : CLOUD_EDGE_EPS;
-        o.risky = entry_edge(fminf(zrk * zto1, 500.0f), eps) || entry_edge(fminf(zto1 / prmuz, 500.0f), eps);
+        o.risky = entry_edge(fminf(zrk * zto1, 500.0f), eps) || entry_edge(fminf(quot(zto1, prmuz), 500.0f), eps);
     }
-    const float p1 = om1 / zem1;  // zep1 - 1
-    const float p2 = om2 / zem2;  // zep2 - 1
+    const float p1 = quot(om1, zem1);  // zep1 - 1
+    const float p2 = quot(om2, zem2);  // zep2 - 1
     const float zdenr = zrpp * (zrk2 + zrkg * p1 + g2k * om1);
     if (zdenr >= -eps && zdenr <= eps) {
         o.ref = eps;
