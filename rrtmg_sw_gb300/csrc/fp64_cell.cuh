@@ -26,10 +26,10 @@
 //     the diffuse flux below a layer follows from the fluxes above it through
 //     the division that the up-sweep has done already.
 //
-// About 168 FP64 instructions per cell (with aerosol; without, a dozen fewer
+// About 167 FP64 instructions per cell (with aerosol; without, a dozen fewer
 // in the layer solution alone: gamma3 = gamma4 = 1/2 and one alpha) where the
 // reference's order of operations took about 570: 16 384 x 60 columns with
-// clouds and aerosol 102.9 -> 36.8 ms, 4 096 x 60 with clouds 28.2 -> 8.4 ms,
+// clouds and aerosol 102.9 -> 36.3 ms, 4 096 x 60 with clouds 28.2 -> 8.4 ms,
 // the FP64 pipe 84 % busy.  The layer solution is also written without the cancellation of
 // thin layers: against a solve in 80-bit arithmetic the heating rates of
 // 1 024 x 60 clear columns are 8.6e-11 off (2-norm), 1.04e-10 in the
@@ -314,9 +314,20 @@ __device__ __forceinline__ Rt64 two_stream64(double tau, double s, double sg, do
         if (__double_as_longlong(e2) == __double_as_longlong(1.0)) { o.ref = 0.0; o.refd = 0.0; o.trad = 1.0; o.tdif = 0.0; }
         return o;
     }
-    const double h = fma(-0.25, w, G ? fma(-0.75, wg, 1.0) : 1.0);  // (gamma1 + gamma2) / 2
-    const double g1 = h + co, g2 = h - co;
-    const double k = sqrt64(4.0 * co * h);
+    // h: gamma1 - gamma2 with asymmetry, half of gamma1 + gamma2 without
+    double h, g1, g2, k;
+    if constexpr (G) {
+        const double sum = fma(-0.5, w, fma(-1.5, wg, 2.0));
+        h = co + co;
+        g1 = fma(0.5, sum, co);
+        g2 = fma(0.5, sum, -co);
+        k = sqrt64(h * sum);
+    } else {
+        h = fma(-0.25, w, 1.0);
+        g1 = h + co;
+        g2 = h - co;
+        k = sqrt64(4.0 * co * h);
+    }
     const double kmu = k * m.mu;
     const double p1 = 1.0 + kmu, m1 = 1.0 - kmu;
     const double pp = p1 * m1;  // 1 - (k mu0)^2
@@ -335,7 +346,7 @@ __device__ __forceinline__ Rt64 two_stream64(double tau, double s, double sg, do
     // Without asymmetry gamma3 = gamma4 = 1/2, alpha1 = alpha2 = h.
     double r3, t3, r2o, t2o;  // zr3, zt3, zr2 oo, zt2 oo
     if constexpr (G) {
-        const double a1 = fma(g2, g3, g1 * g4), a2 = fma(g1, g3, g2 * g4);
+        const double a1 = fma(-h, g3, g1), a2 = fma(h, g3, g2);
         r3 = fma(-a2, m.mu, g3);
         t3 = fma(a1, m.mu, g4);
         r2o = p1 * fma(-k, g3, a2) * oo;
