@@ -1073,8 +1073,10 @@ int solve_static(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cu
     LaunchInfo li = fp32 ? plan_fp32(P, st.num_sms, !st.no_tiled) : plan_fp64(P, st.num_sms);
     // the tiled kernel's prepared blocks (one per pair) must fit beside its
     // per-CTA areas; larger calls take the scratch-based kernel
+    auto over = [&]() { return ovf_offset((size_t)li.grid * li.slot_bytes) + (size_t)P.npairs * li.prep_bytes > avail; };
+    if (li.tiled && over()) li.slot_bytes = li.slot_bytes_min;
+    if (li.tiled && over()) li = plan_fp32(P, st.num_sms, false);
     const size_t off_prep = (((size_t)li.grid * li.slot_bytes) + 255) & ~(size_t)255;
-    if (li.tiled && off_prep + (size_t)P.npairs * li.prep_bytes > avail) li = plan_fp32(P, st.num_sms, false);
     st.last_kernel = !fp32 ? RRTMG_SW_KERNEL_FP64 : li.tiled ? RRTMG_SW_KERNEL_FP32_TILED : RRTMG_SW_KERNEL_FP32;
     st.last_tile_slots = fp32 && li.tiled ? li.tile_slots : 0;
     // one slot per SM, or per column pair when the call has fewer pairs, of

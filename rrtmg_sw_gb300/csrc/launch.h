@@ -14,6 +14,7 @@ struct LaunchInfo {
     size_t smem;         // dynamic shared memory per CTA
     bool tiled = false;  // FP32 form: the tiled kernel (layer R/T in shared memory)
     size_t slot_bytes = 0;  // global scratch per CTA
+    size_t slot_bytes_min = 0;  // tiled kernel: without the pair's cloud optics (each cell computes its own)
     // tiled kernel: its preparation kernel's grid and shared memory, and the
     // bytes of one pair's prepared block (P.tprep holds npairs of them)
     int prep_grid = 0;

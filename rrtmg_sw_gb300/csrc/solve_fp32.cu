@@ -229,7 +229,8 @@ LaunchInfo plan_fp32(const SolveParams& P, int num_sms, bool allow_tiled) {
         cudaFuncSetAttribute(tiled_kernel(P), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)li.smem);
         li.grid = num_sms < P.npairs ? num_sms : P.npairs;
         if (li.grid < 1) li.grid = 1;
-        li.slot_bytes = tiled_glob(P.nlay).total;
+        li.slot_bytes = tiled_glob(P.nlay, fused && P.iaer == 0).total;
+        li.slot_bytes_min = tiled_glob(P.nlay, false).total;
         // the preparation kernel: persistent over the pairs at the occupancy it reaches
         li.prep_smem = tiled_prep_smem(P.nlay).total;
         li.prep_bytes = tiled_prep_layout(P.nlay, fused, fused || nomc, P.iaer != 0).total;

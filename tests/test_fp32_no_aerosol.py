@@ -4,7 +4,9 @@ multiplies by zero and by one: both calls must give the same result.
 
 Tolerance 0: the two instances round the same products and sums.  Sizes: a
 lone column, a half-empty pair, fewer and more pairs than SMs; clear sky,
-random and overlapping McICA clouds, all outputs.
+random and overlapping McICA clouds, all outputs.  That instance also works
+out the cloud optics once per (column, layer, band): layers without a cloudy
+subcolumn must not be looked at, as before (their inputs may be anything).
 """
 import numpy as np
 import pytest
@@ -49,3 +51,31 @@ def test_equals_aerosol_of_depth_zero(ncol, nlay, icld, outputs):
     for k in a:
         if isinstance(a[k], np.ndarray):
             np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+@pytest.mark.parametrize("ncol,nlay", [(5, 60), (333, 33)])
+def test_cloud_inputs_of_clear_layers_are_not_read(ncol, nlay):
+    c = make_columns(ncol, nlay, 5200 + nlay, clouds=True, ptop=0.01)
+    c["alpha"] = np.zeros((ncol, nlay))
+    clear = c["cldfrac"] == 0.0
+    assert clear.any() and not clear.all()
+    for k in ("ciwp", "clwp"):
+        c[k] = np.where(clear, 0.0, c[k])
+    ref = solve(c, 2, 0, False)
+    bad = dict(c)
+    for k, v in (("ciwp", 50.0), ("clwp", 50.0), ("rei", 1.0e4), ("rel", 1.0e4)):
+        bad[k] = np.where(clear, v, c[k])
+    got = solve(bad, 2, 0, False)
+    for k in ref:
+        np.testing.assert_array_equal(got[k], ref[k], err_msg=k)
+    for k, v in (("rei", 1.0e4), ("rel", 1.0e4)):  # and a cloudy layer's still are
+        bad = dict(c)
+        bad["cldfrac"] = np.ones_like(c["cldfrac"])
+        bad["ciwp"] = np.full_like(c["ciwp"], 10.0)
+        bad["clwp"] = np.full_like(c["clwp"], 10.0)
+        bad["rei"] = np.full_like(c["rei"], 30.0)
+        bad["rel"] = np.full_like(c["rel"], 10.0)
+        bad[k] = bad[k].copy()
+        bad[k][ncol // 2, nlay // 2] = v
+        with pytest.raises(gpu.RRTMGError):
+            solve(bad, 2, 0, False)
