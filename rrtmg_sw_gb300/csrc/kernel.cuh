@@ -814,9 +814,9 @@ __device__ inline KissJump kiss_setup(const SolveParams& P, uint32_t* sXs, int g
     return J;
 }
 
-// Column slot and g-point of CTA thread t.  The adjoint (taumol_g runs a
+// Column slot and g-point of CTA thread t.  The tangent (taumol_g runs a
 // different code path per band, in FP64 duals) uses warps of whole bands from
-// two columns (cT.thr_cg over 224 threads); the solves (one
+// two columns (cT.thr_cg over 224 threads); the FP32 solves (one
 // descriptor-driven taumol path, but cloudy layers that differ by column) are
 // faster with 32 consecutive g-points of one column per warp.
 __device__ inline int thread_col_ad(int t) { return cT.thr_cg[t] >> 7; }

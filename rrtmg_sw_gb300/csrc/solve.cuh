@@ -1,6 +1,8 @@
-// solve.cuh -- the fused per-column shortwave solve, templated on the
-// arithmetic type of the bulk work (double: plain FP64 form; float: FP32
-// form).  One CTA handles two columns; each of its 224 threads owns one
+// solve.cuh -- pieces of the fused per-column shortwave solve, templated on
+// the arithmetic type where both precisions use them (double: the reference's
+// order of operations, which the FP32 form and the derivatives take for single
+// cells; the FP64 form's own cell is in fp64_cell.cuh).  The FP32 form's scratch-based
+// kernel: one CTA handles two columns; each of its 224 threads owns one
 // (column, g-point) pair and walks the layers:
 //
 //   prep   (all threads, per column x layer): inatm_sw + setcoef_sw into

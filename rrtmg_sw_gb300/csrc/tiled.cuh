@@ -10,7 +10,8 @@
 // shared memory, two tiles double-buffered.  Warp roles:
 //
 //   optics warps (T_OPT): per pair, the pair's prepared block (below) into
-//     shared memory; then per tile the cells (g-point, layer) -- gas optics, clouds, aerosol,
+//     shared memory and, in calls without aerosol, the cloud optics of its
+//     cloudy (layer, band)s; then per tile the cells (g-point, layer) -- gas optics, clouds, aerosol,
 //     delta scaling, the two-stream layer solution -- layer rows taken from
 //     a shared counter, the 32 subcolumns of a row in one warp (32
 //     consecutive g-points: coalesced table reads).
