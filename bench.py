@@ -663,7 +663,7 @@ def main():
                                                                  % PROFILED_PREP_DRAM_BYTES_PER_COLUMN
                                                                  if kernel == "fp32 tiled" else ""),
                         "time_source": "CUDA events over whole steps (the tiled form's step is its preparation "
-                                       "kernel, ~6 %, and its solve kernel)",
+                                       "kernel, ~9 %, and its solve kernel)",
                         "peak_source": "cuBLAS FP32 (non-TF32) 8192^3 GEMM measured in this run",
                         "flops_per_column": fl, "cloudy_cells_per_column": cloudy}
     line["roofline_hbm"] = {"bound": "hbm", "achieved": bytes_col * ncol / (ms32 / 1e3) / 1e9, "peak": hbm,
