@@ -52,9 +52,10 @@ struct State {
     double mgavgcyc[134], sbavgcyc[134];
     double cpdair = 1.004e3;
     DevBuf d_tab64, d_tab32, scratch, errw, bounds;
+    DevBuf errw64;                         // FP64 device solves' error word, zero between calls
     std::map<std::string, DevBuf> stage;  // host-API staging buffers
-    int* h_err = nullptr;                  // pinned: error word (device solves write it directly)
-    unsigned long long* h_stats = nullptr;  // pinned: the FP32 form's counters of the last solve, overflow count
+    int* h_err = nullptr;                  // pinned: error code of the last call
+    unsigned long long* h_stats = nullptr;  // pinned: the FP32 form's counters of the last solve, overflow count, error word
     DevBuf statsw;                         // their device copy
     long long last_stats[4] = {0, 0, 0, 0};
     // from the environment at each rrtmg_sw_ini_c: RRTMG_SW_TILED=0 keeps the
@@ -585,11 +586,12 @@ size_t ovf_bytes(int npairs) { return (size_t)(npairs + 1) * sizeof(int); }
 // buffer and device error word; nothing is synchronised.  Pout / liout
 // receive the parameters and launch shape (the tiled FP32 kernel's overflow
 // list is read by the caller).  ovf_count: a zeroed device word for the
-// tiled kernel's overflow count (nullptr: one in the scratch, zeroed here).
+// tiled kernel's overflow count (nullptr: one in the scratch, zeroed here);
+// err_host: launch_solve_fp64's.
 int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cudaStream_t s, bool nomcica,
                   DevBuf& scratch, int* err, int& launches, SolveParams* Pout = nullptr,
                   LaunchInfo* liout = nullptr, bool allow_tiled = true, unsigned long long* stats = nullptr,
-                  int* ovf_count = nullptr) {
+                  int* ovf_count = nullptr, int* err_host = nullptr) {
     SolveParams P;
     int rc = make_params(st, a, c, P, nomcica);
     if (rc) return rc;
@@ -628,7 +630,7 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
         launches += 1;  // the preparation kernel
     }
     if (fp32) CK(launch_solve_fp32(P, (const float*)st.d_tab32.p, (const double*)st.d_tab64.p, li, s));
-    else CK(launch_solve_fp64(P, (const double*)st.d_tab64.p, li, s));
+    else CK(launch_solve_fp64(P, (const double*)st.d_tab64.p, li, s, err_host));
     if (Pout) *Pout = P;
     if (liout) *liout = li;
     return RRTMG_SW_OK;
@@ -678,32 +680,49 @@ int tiled_fallback(State& st, const SolveParams& Pt, int count, cudaStream_t s, 
 
 // Queue one solve on `s`; returns with its error word (and, after the tiled
 // FP32 kernel, after solving again any column pairs it could not finish).
-// The kernels write the error word to page-locked host memory themselves;
-// the FP32 form's counters and the tiled kernel's overflow count share one
-// device buffer, zeroed and read back once.  With a memset and a copy for each
-// (and a second synchronisation for the counters), a call of one column spent
-// as long on them as on its kernels.
+// The FP32 form's counters, the tiled kernel's overflow count and the error
+// word share one device buffer, zeroed and read back once.  With a memset and
+// a copy for each (and a second synchronisation for the counters), a call of
+// one column spent as long on them as on its kernels.  The FP64 form's error
+// word is zero between calls (a call that fails clears it), and the split
+// kernels leave it in page-locked memory.  The kernels' atomics stay on the
+// device word: on a word in host memory each is a trip over the link, and a
+// call of 4 096 x 60 columns with every cloud radius out of range took 337 ms
+// (a valid one 43; now 43).
 int solve_dev(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, cudaStream_t s, bool nomcica = false,
               bool allow_tiled = true) {
-    volatile int* err = st.h_err;
-    *err = 0;
     int launches = 0;
     SolveParams P;
     LaunchInfo li;
     const bool fp32 = st.form == RRTMG_SW_FORM_FP32;
-    unsigned long long* words = nullptr;  // 4 counters, then the overflow count
-    constexpr size_t kWords = 5 * sizeof(unsigned long long);
-    for (int i = 0; i < 5; ++i) st.h_stats[i] = 0;
+    unsigned long long* words = nullptr;  // 4 counters, the overflow count, the error word
+    constexpr size_t kWords = 6 * sizeof(unsigned long long);
+    for (int i = 0; i < 6; ++i) st.h_stats[i] = 0;
+    int* word = (int*)st.errw64.p;
+    volatile int* err = st.h_err;
+    *err = 0;
     if (fp32) {
         CK(st.statsw.ensure(kWords));
         words = (unsigned long long*)st.statsw.p;
         CK(cudaMemsetAsync(words, 0, kWords, s));
+        word = (int*)(words + 5);
+        err = (volatile int*)(st.h_stats + 5);
     }
-    const int rc = enqueue_solve(st, a, c, s, nomcica, st.scratch, st.h_err, launches, &P, &li, allow_tiled, words,
-                                 fp32 ? (int*)(words + 4) : nullptr);
-    if (rc) return rc;
+    const int rc = enqueue_solve(st, a, c, s, nomcica, st.scratch, word, launches, &P, &li, allow_tiled, words,
+                                 fp32 ? (int*)(words + 4) : nullptr, fp32 ? nullptr : st.h_err);
+    auto clear_word = [&]() {  // FP64: after the kernels of a call that failed
+        cudaStreamSynchronize(s);
+        cudaMemsetAsync(word, 0, sizeof(int), s);
+        cudaStreamSynchronize(s);
+    };
+    if (rc) {
+        if (rc == RRTMG_SW_ECUDA && !fp32) clear_word();
+        return rc;
+    }
     if (fp32) CK(cudaMemcpyAsync(st.h_stats, words, kWords, cudaMemcpyDeviceToHost, s));
+    else if (!li.split_lb) CK(cudaMemcpyAsync(st.h_err, word, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (*err && !fp32) clear_word();
     const int ovf = (int)st.h_stats[4];
     if (li.tiled && *err == 0 && ovf > 0) {
         DevBuf& cm = st.stage["tovf_colmap"];
@@ -1402,7 +1421,9 @@ int rrtmg_sw_ini_c(double cpdair) {
         const int rc = build_tables(st);
         if (rc) return rc;
         CK(cudaMallocHost((void**)&st.h_err, sizeof(int)));
-        CK(cudaMallocHost((void**)&st.h_stats, 5 * sizeof(unsigned long long)));
+        CK(cudaMallocHost((void**)&st.h_stats, 6 * sizeof(unsigned long long)));
+        CK(st.errw64.ensure(sizeof(int)));
+        CK(cudaMemset(st.errw64.p, 0, sizeof(int)));
         CK(cudaStreamCreateWithFlags(&st.host_stream, cudaStreamNonBlocking));
     }
     {
@@ -1757,6 +1778,7 @@ int rrtmg_sw_finalize_c(void) {
     st.d_tab32.release();
     st.scratch.release();
     st.errw.release();
+    st.errw64.release();
     st.statsw.release();
     st.bounds.release();
     for (auto& kv : st.stage) kv.second.release();

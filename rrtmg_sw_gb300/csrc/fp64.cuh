@@ -517,9 +517,12 @@ __host__ __device__ inline SweepSmem64 sweep_smem64(const SolveParams& P) {
 
 // Sweeps of column blockIdx.x, sky blockIdx.y (0 clear, 1 total; a clear call
 // has one sky and writes both skies' outputs), g-point sums and outputs.
+// err_host: where one thread leaves the error word, which only k_cells64
+// writes; a copy of its own would cost a small call a few microseconds.
 __global__ void __launch_bounds__(SWEEP_THREADS)
-k_sweep64(const SolveParams P, const double* __restrict__ tab) {
+k_sweep64(const SolveParams P, const double* __restrict__ tab, int* err_host) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (err_host && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *(volatile int*)err_host = *P.err;
     constexpr int NT = CTA_THREADS;
     const SweepSmem64 M = sweep_smem64(P);
     int* pk = (int*)(smem_raw + M.pk);

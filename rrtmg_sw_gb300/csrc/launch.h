@@ -26,7 +26,9 @@ struct LaunchInfo {
 // FP64 form
 cudaError_t upload_tables_fp64(const DevTables& t);
 LaunchInfo plan_fp64(const SolveParams& P, int num_sms, bool allow_split = true);
-cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s);
+// err_host (page-locked, nullptr: none): the split kernels leave the error word there too
+cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s,
+                              int* err_host = nullptr);
 // FP32 form
 cudaError_t upload_tables_fp32(const DevTables& t);
 // setcoef of the FP32 form (FP32 arithmetic, the FP64 form's indices) over all (column, layer)

@@ -57,7 +57,8 @@ LaunchInfo plan_fp64(const SolveParams& P, int num_sms, bool allow_split) {
     return li;
 }
 
-cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s) {
+cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const LaunchInfo& li, cudaStream_t s,
+                              int* err_host) {
     if (li.split_lb) {
         const size_t sc = split_smem64(P).total, ss = sweep_smem64(P).total;
         const auto cells = P.mt ? k_cells64<true> : k_cells64<false>;
@@ -66,7 +67,7 @@ cudaError_t launch_solve_fp64(const SolveParams& P, const double* tab, const Lau
         if (e != cudaSuccess) return e;
         const dim3 gc(P.npairs, (P.nlay + li.split_lb - 1) / li.split_lb), gs(P.ncol, cloud_mode(P) == CLD_NONE ? 1 : 2);
         cells<<<gc, SPLIT_THREADS, sc, s>>>(P, li.split_lb, tab);
-        k_sweep64<<<gs, SWEEP_THREADS, ss, s>>>(P, tab);
+        k_sweep64<<<gs, SWEEP_THREADS, ss, s>>>(P, tab, err_host);
         return cudaGetLastError();
     }
     if (P.mt) k_solve64<true><<<li.grid, CTA_THREADS, li.smem, s>>>(P, tab);
