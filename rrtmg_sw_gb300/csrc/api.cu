@@ -612,12 +612,30 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
     LaunchInfo li = fp32 ? plan_fp32(P, st.num_sms, allow_tiled && !st.no_tiled) : plan_fp64(P, st.num_sms);
     st.last_kernel = !fp32 ? RRTMG_SW_KERNEL_FP64 : li.tiled ? RRTMG_SW_KERNEL_FP32_TILED : RRTMG_SW_KERNEL_FP32;
     st.last_tile_slots = fp32 && li.tiled ? li.tile_slots : 0;
-    P.slot_elems = li.slot_bytes / (fp32 ? sizeof(float) : sizeof(double));
-    if (li.split_lb) launches += 1;  // cells, then sweeps
     // tiled: per-CTA areas, then the pairs' prepared blocks, then the overflow list
     const size_t off_prep = ovf_offset((size_t)li.grid * li.slot_bytes);
     const size_t off = ovf_offset(off_prep + (size_t)P.npairs * li.prep_bytes);
-    CK(scratch.ensure(li.tiled ? off + ovf_bytes(P.npairs) : (size_t)li.grid * li.slot_bytes));
+    size_t need = li.tiled ? off + ovf_bytes(P.npairs) : (size_t)li.grid * li.slot_bytes;
+    // the split FP64 kernels want a slot per column pair; where the memory is
+    // short the fused kernel makes do with one per resident CTA
+    auto fused = [&]() {
+        li = plan_fp64(P, st.num_sms, false);
+        need = (size_t)li.grid * li.slot_bytes;
+    };
+    if (li.split_lb && need > scratch.bytes) {
+        size_t fr = 0, tot = 0;
+        CK(cudaMemGetInfo(&fr, &tot));
+        if (need > scratch.bytes + fr) fused();
+    }
+    cudaError_t e = scratch.ensure(need);
+    if (e == cudaErrorMemoryAllocation && li.split_lb) {
+        cudaGetLastError();
+        fused();
+        e = scratch.ensure(need);
+    }
+    CK(e);
+    P.slot_elems = li.slot_bytes / (fp32 ? sizeof(float) : sizeof(double));
+    if (li.split_lb) launches += 1;  // cells, then sweeps
     P.scratch = scratch.p;
     if (li.tiled) {
         P.tprep = (char*)scratch.p + off_prep;
