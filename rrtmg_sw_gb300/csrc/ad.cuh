@@ -721,26 +721,33 @@ __device__ inline void prep_band_deriv(const SolveParams& P, int pcol, int lay, 
     if (mode == CLD_MASK) {
         const size_t kl = (size_t)pcol + (size_t)P.ncol * (size_t)(lay - 1);
         if (P.cldfrac[kl] > 0.0) {
-            // the optics are sums of a liquid and an ice part, each
-            // proportional to its water path (fixed when inflgsw = 0)
+            // the optics are sums of a liquid and an ice part, each its
+            // optics per unit of water path times the path (fixed when
+            // inflgsw = 0, zero where a part has no path or no
+            // parametrisation: cloud64 then puts its floor of 1e-20 there)
             const double wl = P.clwp[kl], wi = P.ciwp[kl];
-            double c[CO_N];
             double* o = cj + b * CJ_N;
-            const bool on = P.inflag == 2 && wl + wi >= 1.e-20;
             for (int k = 0; k < CJ_N; ++k) o[k] = 0.0;
-            if (on && wl >= 1.e-20) {
-                cloud64(b, P.inflag, P.iceflag, P.liqflag, 1.0, 0.0, wl, P.rei[kl], P.rel[kl], 0.0, 0.0, 1.0, 0.0, tab,
+            const bool on = P.inflag == 2 &&
+                            (wl + wi >= 1.e-20 || (P.tauc && P.tauc[(size_t)b + 14 * kl] >= 1.e-20));
+            double c[CO_N];
+            if (on && wl != 0.0) {
+                cloud64(b, P.inflag, P.iceflag, P.liqflag, 1.0, 0.0, 1.0, P.rei[kl], P.rel[kl], 0.0, 0.0, 1.0, 0.0, tab,
                         -1.0, c);
-                o[CJ_SL] = c[CO_S] / wl;
-                o[CJ_GL] = c[CO_SG] / wl;
-                o[CJ_AL] = c[CO_AB] / wl;
+                if (c[CO_TAU] > 1.e-20) {
+                    o[CJ_SL] = c[CO_S];
+                    o[CJ_GL] = c[CO_SG];
+                    o[CJ_AL] = c[CO_AB];
+                }
             }
-            if (on && wi >= 1.e-20) {
-                cloud64(b, P.inflag, P.iceflag, P.liqflag, 1.0, wi, 0.0, P.rei[kl], P.rel[kl], 0.0, 0.0, 1.0, 0.0, tab,
+            if (on && wi != 0.0) {
+                cloud64(b, P.inflag, P.iceflag, P.liqflag, 1.0, 1.0, 0.0, P.rei[kl], P.rel[kl], 0.0, 0.0, 1.0, 0.0, tab,
                         -1.0, c);
-                o[CJ_SI] = c[CO_S] / wi;
-                o[CJ_GI] = c[CO_SG] / wi;
-                o[CJ_AI] = c[CO_AB] / wi;
+                if (c[CO_TAU] > 1.e-20) {
+                    o[CJ_SI] = c[CO_S];
+                    o[CJ_GI] = c[CO_SG];
+                    o[CJ_AI] = c[CO_AB];
+                }
             }
         }
     }
