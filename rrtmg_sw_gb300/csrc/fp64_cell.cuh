@@ -369,7 +369,9 @@ __device__ __forceinline__ Rt64 two_stream64(double tau, double s, double sg, do
 // Cloud optics of a layer in band ib (cldprmc_sw, rrtmg_sw_cldprmc.f90:53-349;
 // with ttest >= 0 cldprop_sw's test) in the form two_stream64 takes.  The
 // error code of an input out of range is returned in c[CO_ERR]: it counts
-// only where a cloudy subcolumn meets it.
+// only where a cloudy subcolumn meets it.  A radius that is no number counts as
+// out of range: the preparation comes here for every layer that may be cloudy
+// (with MT19937 for all), and some callers leave NaN where there is no cloud.
 __device__ inline void cloud64(int ib, int inflag, int iceflag, int liqflag, double cldf, double ciwp, double clwp,
                                double rei, double rel, double fsfc, double tauc, double ssac, double asmc,
                                const double* __restrict__ tab, double ttest, double* c) {
@@ -404,7 +406,7 @@ __device__ inline void cloud64(int ib, int inflag, int iceflag, int liqflag, dou
     };
     auto bad = [](double e, double s, double g) { return e < 0.0 || s > 1.0 || s < 0.0 || g > 1.0 || g < 0.0; };
     if (ciwp != 0.0 && iceflag == 1) {
-        if (rei < 13.0 || rei > 130.0) { err = E_ICERAD; out(); return; }
+        if (!(rei >= 13.0 && rei <= 130.0)) { err = E_ICERAD; out(); return; }
         const double w2 = ldt(tab, cT.wavenum2 + ib);
         const int icx = w2 > 1.43e04 ? 1 : w2 > 7.7e03 ? 2 : w2 > 5.3e03 ? 3 : w2 > 4.0e03 ? 4 : w2 >= 2.5e03 ? 5 : 0;
         exti = ldt(tab, cT.abari + icx - 1) + ldt(tab, cT.bbari + icx - 1) / rei;
@@ -415,7 +417,7 @@ __device__ inline void cloud64(int ib, int inflag, int iceflag, int liqflag, dou
         fwi = gi * gi;
         if (bad(exti, ssai, gi)) { err = E_ICEPROP; out(); return; }
     } else if (ciwp != 0.0 && iceflag == 2) {
-        if (rei < 5.0 || rei > 131.0) { err = E_ICERAD; out(); return; }
+        if (!(rei >= 5.0 && rei <= 131.0)) { err = E_ICERAD; out(); return; }
         const double factor = (rei - 2.0) / 3.0;
         int index = (int)factor;
         if (index == 43) index = 42;
@@ -427,7 +429,7 @@ __device__ inline void cloud64(int ib, int inflag, int iceflag, int liqflag, dou
         fwi = gi * gi;
         if (bad(exti, ssai, gi)) { err = E_ICEPROP; out(); return; }
     } else if (ciwp != 0.0 && iceflag == 3) {
-        if (rei < 5.0 || rei > 140.0) { err = E_ICEDGE; out(); return; }
+        if (!(rei >= 5.0 && rei <= 140.0)) { err = E_ICEDGE; out(); return; }
         const double factor = (rei - 2.0) / 3.0;
         int index = (int)factor;
         if (index == 46) index = 45;
@@ -443,7 +445,7 @@ __device__ inline void cloud64(int ib, int inflag, int iceflag, int liqflag, dou
         if (bad(exti, ssai, gi)) { err = E_ICEPROP; out(); return; }
     }
     if (clwp != 0.0 && liqflag == 1) {
-        if (rel < 2.5 || rel > 60.0) { err = E_LIQRAD; out(); return; }
+        if (!(rel >= 2.5 && rel <= 60.0)) { err = E_LIQRAD; out(); return; }
         int index = (int)(rel - 1.5);
         if (index == 0) index = 1;
         if (index == 58) index = 57;
