@@ -138,10 +138,6 @@ template <> __device__ inline Dual<5> c_oneminus<Dual<5>>() { return Dual<5>(cT.
 template <> __device__ inline Dual<3> c_bpade<Dual<3>>() { return Dual<3>(cT.bpade); }
 template <> __device__ inline Dual<5> c_bpade<Dual<5>>() { return Dual<5>(cT.bpade); }
 
-__device__ inline double val(double x) { return x; }
-template <int N>
-__device__ inline double val(const Dual<N>& x) { return x.v; }
-
 // Dual<5> holding the value and derivatives of a Dual<3> in its first slots
 __device__ inline Dual<5> widen(const Dual<3>& a) {
     Dual<5> r(a.v);
@@ -347,12 +343,10 @@ __device__ inline void cell_total(const CellIn<T>& ci, double prmu0, T out[5]) {
 // water-path derivatives.  Each variant is compiled once (not inlined at
 // its call sites): the kernel's instruction footprint, not its arithmetic,
 // was what its warps waited on most.
-__device__ inline Dual<5> widen5(const Dual<3>& a) { return widen(a); }
-
 __device__ __noinline__ void ad_cell_clear(const CellIn<Dual<3>>& ci, double cossza, Dual<5> out[5]) {
     Dual<3> o[5];
     cell_total(ci, cossza, o);
-    for (int k = 0; k < 5; ++k) out[k] = widen5(o[k]);
+    for (int k = 0; k < 5; ++k) out[k] = widen(o[k]);
 }
 
 __device__ __noinline__ void ad_cell_cloudy(const SolveParams& P, const CellIn<Dual<3>>& c3, int col, int lay, int ib,
@@ -360,9 +354,9 @@ __device__ __noinline__ void ad_cell_cloudy(const SolveParams& P, const CellIn<D
                                             const double* __restrict__ tab64, Dual<5> out[5]) {
     typedef Dual<5> D;
     CellIn<D> ci;
-    ci.taug = widen5(c3.taug);
-    ci.taur = widen5(c3.taur);
-    ci.rta = widen5(c3.rta); ci.roa = widen5(c3.roa); ci.rga = widen5(c3.rga); ci.rcoa = widen5(c3.rcoa);
+    ci.taug = widen(c3.taug);
+    ci.taur = widen(c3.taur);
+    ci.rta = widen(c3.rta); ci.roa = widen(c3.roa); ci.rga = widen(c3.rga); ci.rcoa = widen(c3.rcoa);
     ci.cloudy = true;
     ci.cldf = D(1.0);
     D ciwp(cld[0 * L + lay - 1]), clwp(cld[1 * L + lay - 1]);
