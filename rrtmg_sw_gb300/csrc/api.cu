@@ -69,6 +69,8 @@ struct State {
     // host-array calls run on this non-blocking stream (not the legacy
     // default stream, which would serialise against every stream of the host)
     cudaStream_t host_stream = nullptr;
+    cudaStream_t ad_stream = nullptr;  // the tangent-linear's J, beside its dJ on host_stream
+    cudaEvent_t ad_event[2] = {nullptr, nullptr};
     int form = RRTMG_SW_FORM_FP64;
     int last_launches = 0;
     int last_kernel = -1;  // RRTMG_SW_KERNEL_* of the most recent solve's main launch
@@ -1234,7 +1236,7 @@ int solve_ad_host(const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, const rrtmg_
         // (beyond what is already allocated), else recomputed
         size_t fr = 0, tot = 0;
         CK(cudaMemGetInfo(&fr, &tot));
-        const size_t need = plan_adjoint(P, A.tl, 1, st.num_sms).scratch;
+        const size_t need = plan_adjoint(P, 0, 1, st.num_sms).scratch;
         A.store = need <= st.scratch.bytes + fr / 2 ? 1 : 0;
     }
     st.last_ad_store = A.store;
@@ -1242,7 +1244,20 @@ int solve_ad_host(const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, const rrtmg_
     CK(st.scratch.ensure(plan.scratch));
     P.scratch = st.scratch.p;
     CK(cudaMemsetAsync(P.err, 0, sizeof(int), s));
-    CK(launch_adjoint(P, A, (const double*)st.d_tab64.p, plan, s));
+    if (tl) {
+        // J beside dJ: on the SMs that a call of few columns leaves idle, else
+        // where k_tangent's last column pairs run out (launched first it would
+        // keep some of k_tangent's CTAs waiting for it)
+        CK(cudaEventRecord(st.ad_event[0], s));
+        CK(cudaStreamWaitEvent(st.ad_stream, st.ad_event[0], 0));
+        CK(launch_tangent(P, A, (const double*)st.d_tab64.p, plan, s));
+        const cudaError_t e = launch_adjoint(P, A, (const double*)st.d_tab64.p, plan, st.ad_stream);
+        CK(cudaEventRecord(st.ad_event[1], st.ad_stream));
+        CK(cudaStreamWaitEvent(s, st.ad_event[1], 0));
+        CK(e);
+    } else {
+        CK(launch_adjoint(P, A, (const double*)st.d_tab64.p, plan, s));
+    }
     st.last_launches = tl ? 2 : 1;
     sg.back(ad->J, A.J, C);
     if (tl) sg.back(ad->dJ, A.dJ, C);
@@ -1443,6 +1458,8 @@ int rrtmg_sw_ini_c(double cpdair) {
         CK(st.errw64.ensure(sizeof(int)));
         CK(cudaMemset(st.errw64.p, 0, sizeof(int)));
         CK(cudaStreamCreateWithFlags(&st.host_stream, cudaStreamNonBlocking));
+        CK(cudaStreamCreateWithFlags(&st.ad_stream, cudaStreamNonBlocking));
+        for (cudaEvent_t& e : st.ad_event) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     {
         const char* t = std::getenv("RRTMG_SW_TILED");
@@ -1807,6 +1824,12 @@ int rrtmg_sw_finalize_c(void) {
     st.h_stats = nullptr;
     if (st.host_stream) cudaStreamDestroy(st.host_stream);
     st.host_stream = nullptr;
+    if (st.ad_stream) cudaStreamDestroy(st.ad_stream);
+    st.ad_stream = nullptr;
+    for (cudaEvent_t& e : st.ad_event) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
     // a later rrtmg_sw_ini_c (after a cudaDeviceReset, say) looks the static
     // area's address up again
     for (StaticArea& sa : g_static_area) sa = StaticArea{};

@@ -54,14 +54,16 @@ cudaError_t launch_batch_fp32(const SolveParams* dPb, int n, const int* counts, 
 // tangent-linear / adjoint (solve_ad.cu)
 cudaError_t upload_tables_ad(const DevTables& t);
 struct AdPlan {
-    // k_adjoint and, for the tangent-linear, k_tangent before it: CTAs
-    // (persistent over the column pairs), dynamic shared memory and scratch
-    // doubles per CTA; scratch: bytes of the larger one
+    // k_adjoint (for the tangent-linear the instance that forms J alone) and
+    // k_tangent: CTAs (persistent over the column pairs), dynamic shared memory
+    // and scratch doubles per CTA; scratch: bytes of both, the tangent's from
+    // tl_scratch on
     int grid = 0, tl_grid = 0;
-    size_t smem = 0, tl_smem = 0, slot_elems = 0, tl_slot_elems = 0, scratch = 0;
+    size_t smem = 0, tl_smem = 0, slot_elems = 0, tl_slot_elems = 0, tl_scratch = 0, scratch = 0;
 };
 AdPlan plan_adjoint(const SolveParams& P, int tl, int store, int num_sms);
 cudaError_t launch_adjoint(SolveParams P, const AdParams& A, const double* tab64, const AdPlan& a, cudaStream_t s);
+cudaError_t launch_tangent(SolveParams P, const AdParams& A, const double* tab64, const AdPlan& a, cudaStream_t s);
 // scratch elements per CTA slot of nc columns: of the scratch-based kernels'
 // type (also the size by which rrtmg_sw_static_dev_c refuses a call in either
 // form), and doubles of the FP64 form (fewer than the former)

@@ -21,27 +21,32 @@ static int resident_grid(K kern, size_t smem, int npairs, int num_sms) {
 
 AdPlan plan_adjoint(const SolveParams& P, int tl, int store, int num_sms) {
     AdPlan a;
-    a.smem = ad_smem(P.nlay, COLS_PER_CTA).total;
-    a.slot_elems = ad_slot(P.nlay, store, COLS_PER_CTA).total;
-    a.grid = resident_grid(k_adjoint<COLS_PER_CTA>, a.smem, P.npairs, num_sms);
+    const auto kern = tl ? k_adjoint<COLS_PER_CTA, true> : k_adjoint<COLS_PER_CTA, false>;
+    a.smem = ad_smem(P.nlay, COLS_PER_CTA, tl != 0).total;
+    a.slot_elems = ad_slot(P.nlay, tl ? AD_J : store, COLS_PER_CTA).total;
+    a.grid = resident_grid(kern, a.smem, P.npairs, num_sms);
     a.scratch = (size_t)a.grid * a.slot_elems * sizeof(double);
     if (tl) {
         a.tl_smem = tl_smem_layout(P.nlay).total;
         a.tl_slot_elems = tl_slot_elems(P.nlay);
         a.tl_grid = resident_grid(k_tangent, a.tl_smem, P.npairs, num_sms);
-        const size_t need = (size_t)a.tl_grid * a.tl_slot_elems * sizeof(double);
-        if (need > a.scratch) a.scratch = need;
+        a.tl_scratch = a.scratch;
+        a.scratch += (size_t)a.tl_grid * a.tl_slot_elems * sizeof(double);
     }
     return a;
 }
 
 cudaError_t launch_adjoint(SolveParams P, const AdParams& A, const double* tab64, const AdPlan& a, cudaStream_t s) {
-    if (A.tl) {
-        P.slot_elems = a.tl_slot_elems;
-        k_tangent<<<a.tl_grid, CTA_THREADS, a.tl_smem, s>>>(P, A, tab64);
-    }
     P.slot_elems = a.slot_elems;
-    k_adjoint<COLS_PER_CTA><<<a.grid, CTA_THREADS, a.smem, s>>>(P, A, tab64);
+    if (A.tl) k_adjoint<COLS_PER_CTA, true><<<a.grid, CTA_THREADS, a.smem, s>>>(P, A, tab64);
+    else k_adjoint<COLS_PER_CTA, false><<<a.grid, CTA_THREADS, a.smem, s>>>(P, A, tab64);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tangent(SolveParams P, const AdParams& A, const double* tab64, const AdPlan& a, cudaStream_t s) {
+    P.scratch = (char*)P.scratch + a.tl_scratch;
+    P.slot_elems = a.tl_slot_elems;
+    k_tangent<<<a.tl_grid, CTA_THREADS, a.tl_smem, s>>>(P, A, tab64);
     return cudaGetLastError();
 }
 
