@@ -595,6 +595,7 @@ k_tangent(const SolveParams P, const AdParams A, const double* __restrict__ tab6
 // of the FP64 tables: exp(-x) for 0 <= x <= 500 with n = rint(1024 x / ln 2),
 // exp(-x) = 2^(-n/1024) (1 + q), q = expm1(r), r = n ln 2 / 1024 - x, |r| <
 // 3.4e-4 (table-driven, Tang 1989), and om = 1 - exp(-x) without cancellation.
+// exp(-x) is within 2 ulp, om within 4.
 constexpr int EXP2_N = 1024;
 __device__ __forceinline__ void expm64(double x, const double* __restrict__ tab, double& e, double& om) {
     const double magic = 6755399441055744.0;  // 1.5 * 2^52
@@ -609,6 +610,16 @@ __device__ __forceinline__ void expm64(double x, const double* __restrict__ tab,
     const double T = __hiloint2double(__double2hiint(T0) - (m << 20), __double2loint(T0));
     e = fma(T, q, T);
     om = m == 0 ? fma(-T, q, ldt(tab, cT.exp2 + 2 * j + 1)) : 1.0 - e;
+}
+
+// sqrt64 with the reciprocal root: x^1/2 and x^-1/2 for positive normal x, both
+// with an error below 1.1 ulp.
+__device__ __forceinline__ void root64(double x, double& k, double& rk) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double m = x * y, e = fma(-m, y, 1.0), p = e * fma(0.375, e, 0.5);
+    k = fma(m, p, m);
+    rk = fma(y, p, y);
 }
 
 // The prepared block's derivative fields, behind fp64_cell.cuh's B_*: of the
@@ -941,14 +952,7 @@ __device__ __noinline__ void sol_forward(double s, double sg, double ab, const M
         out.dbt = o.e2;
         return;
     }
-    {
-        const double X = co * (G ? fma(-3.0, wg, 4.0 - w) : 4.0 - w);
-        double y;
-        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(X));
-        const double mm = X * y, e = fma(-mm, y, 1.0), p = e * fma(0.375, e, 0.5);
-        o.k = fma(mm, p, mm);
-        o.rk = fma(y, p, y);
-    }
+    root64(co * (G ? fma(-3.0, wg, 4.0 - w) : 4.0 - w), o.k, o.rk);
     expm64(clip500(o.k * tau), tab, o.e1, o.om1);
     const Mid x = sol_mid<G>(o, s, sg, ab, m);
     const double pp = x.p1 * x.m1, pB = pp * x.B;

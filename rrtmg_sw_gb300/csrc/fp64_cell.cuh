@@ -9,7 +9,7 @@
 //
 //   - no IEEE division or square root per cell: rcp64 / sqrt64 start from
 //     the hardware's approximation and take one third-order step (3 and 5
-//     FP64 instructions, within an ulp) instead of a division sequence;
+//     FP64 instructions, error about an ulp) instead of a division sequence;
 //   - explicit fma() (the unit is compiled without contraction, so every
 //     kernel that inlines these functions rounds alike, bit for bit);
 //   - what does not depend on the g-point is made once per (column, layer,
@@ -42,8 +42,10 @@
 namespace rrsw {
 
 // ------------------------------------------------------------ arithmetic
-// 1/x for finite normal x: the hardware's approximation r (relative error e,
-// |e| < 2^-19) and one third-order step r (1 + e + e^2), error below an ulp.
+// 1/x for finite normal x with a normal reciprocal: the hardware's
+// approximation r, e = 1 - x r (|e| < 2^-19), and one step of Householder's
+// iteration of third order for r -> 1/x, r (1 + e + e^2) (A. S. Householder,
+// The Numerical Treatment of a Single Nonlinear Equation, 1970); error below an ulp.
 __device__ __forceinline__ double rcp64(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -51,8 +53,9 @@ __device__ __forceinline__ double rcp64(double x) {
     return fma(r, fma(e, e, e), r);
 }
 
-// sqrt(x) for positive normal x: y ~ x^-1/2 from the hardware, e = 1 - x y^2,
-// sqrt(x) = x y (1 + e/2 + 3 e^2 / 8), error below an ulp.
+// sqrt(x) for positive normal x: y ~ x^-1/2 from the hardware, e = 1 - x y^2, and
+// the same iteration for y -> x^-1/2 times x: sqrt(x) = x y (1 + e/2 + 3 e^2 / 8),
+// the binomial series of x y (1 - e)^-1/2; error below 1.1 ulp.
 __device__ __forceinline__ double sqrt64(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
