@@ -92,7 +92,7 @@ def algorithmic_flops_per_column(nlay, cloudy_cells_per_col):
 # (dram__bytes_read.sum + dram__bytes_write.sum) in captures at 32768 columns x
 # 60 layers, McICA icld=5; the traffic is per column pair, so a launch's
 # traffic scales with its columns.
-PROFILED_DRAM_BYTES_PER_COLUMN = {"fp32 scratch": 28.38e9 / 32768,
+PROFILED_DRAM_BYTES_PER_COLUMN = {"fp32 scratch": 28.82e9 / 32768,
                                   "fp32 tiled": (333.538048e6 + 116.518912e6) / 32768}
 # the tiled kernel's preparation kernel (k_tiled_prep), same capture
 PROFILED_PREP_DRAM_BYTES_PER_COLUMN = (223.528704e6 + 208.922880e6) / 32768
@@ -220,7 +220,7 @@ def run_batch(args):
 def adjoint_workload(args, gi, k=3, recompute=True):
     """Adjoint cost: 65536 columns x 60 layers, McICA clouds (icld=2, masks
     frozen), objective TOA up + surface net + heating-rate sum; forward,
-    tangent-linear and adjoint (stored / recomputed local Jacobians) through
+    tangent-linear and adjoint (stored / recomputed intermediates) through
     the host-array C ABI, each timed end to end (best of k after one
     untimed call)."""
     from rrtmg_sw_gb300.synthetic import gcm_inputs, make_columns
@@ -272,12 +272,15 @@ def run_adjoint(args):
         sms = torch.cuda.get_device_properties(0).multi_processor_count
     except Exception:
         pass
-    # per-CTA scratch (doubles) of the adjoint kernel, 3 resident CTAs per SM
-    slot = lambda fields: ((NLAY + 1) * fields * 224 + 2 * 15 * NLAY * 4) * 8 * 3
+    # scratch of the adjoint kernel (doubles per CTA, 2 resident CTAs per SM):
+    # the stored fields of each (layer, g-point); each (column, layer)'s prepared
+    # block (78), cloud optics and their derivatives, aerosol (16 per band),
+    # setcoef in duals (60) and water paths (4); the queue
+    slot = lambda fields: NLAY * (fields * 224 + 2 * (78 + 16 * 14 + 60 + 4) + 112) * 8 * 2
     line = {"metric": "adjoint cost relative to the FP64 forward it differentiates (host-array calls, end to end)",
             "value": r["adjoint_store_vs_fp64_forward"], "unit": "x forward", "n_gpus": 1,
             "higher_is_better": False, "config": {"workload": r["workload"]},
-            "scratch_bytes_store": slot(45) * sms, "scratch_bytes_recompute": slot(20) * sms}
+            "scratch_bytes_store": slot(26) * sms, "scratch_bytes_recompute": slot(19) * sms}
     line.update({k: v for k, v in r.items() if k != "workload"})
     print(json.dumps(line))
 

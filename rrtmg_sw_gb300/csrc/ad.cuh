@@ -24,8 +24,9 @@
 //   top to bottom  the fluxes, the adjoint of the up-sweep, then that of the
 //            layer solution down to its three optical inputs (scattering,
 //            scattering times asymmetry, absorption) and, through the stored
-//            derivatives, to the layer's inputs, summed over g-points in a
-//            fixed order.
+//            derivatives, to the layer's inputs, summed over g-points (the
+//            queued cells below by atomics, in no fixed order: gradients
+//            differ in their last bits from run to run).
 // Like the FP64 solve it is bound by the FP64 pipe.
 //
 // Where the reference's own derivative is dominated by rounding (NOISE_AD
@@ -33,7 +34,7 @@
 // reference's order of operations (five outputs along three to five directions
 // as duals, about 2 000 FP64 instructions): the second pass queues those cells
 // and the CTA then takes them 32 to a warp.  Formed for every cell, as the
-// tangent does: 4 096 x 60 columns with clouds 160 ms; now 37 ms (91 ms with
+// tangent does: 4 096 x 60 columns with clouds 160 ms; now 34.6 ms (91 ms with
 // each warp forming them on the spot, of its 32 lanes those that need it).
 //
 // k_tangent runs the forward model with every cell's Jacobian in duals

@@ -313,7 +313,7 @@ int build_tables(State& st) {
                 if (y >> b & 1u) r ^= T.xs_jump[k - 1][b];
             T.xs_jump[k][j] = r;
         }
-    // thread layout of the solve CTA: warps of whole bands, both columns
+    // thread layout of the tangent's CTA: warps of whole bands, both columns
     // of a band side by side (band sizes 2*ng: 12,24,16,16,20,20,4,20,16,12,12,16,12,24)
     {
         const int seg[][3] = {  // band, first g in band, count (per column)
@@ -658,7 +658,7 @@ int enqueue_solve(State& st, const rrtmg_sw_args* a, const rrtmg_sw_clouds* c, c
 
 // The tiled FP32 kernel listed `count` column pairs whose FP64 cells
 // exceeded its capacities (their outputs are not final): solve them again
-// with the scratch-based kernel (k_solve<float>, whose FP64 redo has no such
+// with the scratch-based kernel (k_solve, whose FP64 redo has no such
 // limit) through its column map, on the same stream.  With more pairs than
 // the list holds, every pair is solved again.  `colmap` is device memory for
 // 2 * count + 1 ints; `scratch(bytes)` returns device scratch of that size

@@ -10,8 +10,9 @@
 //   - no IEEE division or square root per cell: rcp64 / sqrt64 start from
 //     the hardware's approximation and take one third-order step (3 and 5
 //     FP64 instructions, error about an ulp) instead of a division sequence;
-//   - explicit fma() (the unit is compiled without contraction, so every
-//     kernel that inlines these functions rounds alike, bit for bit);
+//   - explicit fma() (solve_fp64.cu is compiled without contraction, so its
+//     kernels, which all inline these functions, round alike, bit for bit;
+//     the derivatives' unit is not);
 //   - what does not depend on the g-point is made once per (column, layer,
 //     band): the species-ratio interpolation of taumol and the cloud and
 //     aerosol optics (14 bands against 112 g-points);
@@ -26,7 +27,7 @@
 //     the diffuse flux below a layer follows from the fluxes above it through
 //     the division that the up-sweep has done already.
 //
-// About 167 FP64 instructions per cell (with aerosol; without, a dozen fewer
+// 172 FP64 instructions per cell with clouds and aerosol (without aerosol a dozen fewer
 // in the layer solution alone: gamma3 = gamma4 = 1/2 and one alpha) where the
 // reference's order of operations took about 570: 16 384 x 60 columns with
 // clouds and aerosol 102.9 -> 36.3 ms, 4 096 x 60 with clouds 28.2 -> 8.4 ms,

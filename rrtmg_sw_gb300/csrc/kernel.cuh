@@ -803,8 +803,8 @@ __device__ inline void fill_tm(unsigned char* smem_raw) {
 }
 
 // McICA stream jump of subcolumn g (this thread's) for parameters P; the
-// xorshift parts go to sXs (one column of M^n per g-point, filled by the
-// CTA's first 112 threads).
+// xorshift parts go to sXs (the columns of M^n of every g-point, filled by
+// the whole CTA).
 __device__ inline KissJump kiss_setup(const SolveParams& P, uint32_t* sXs, int g) {
     KissJump J{1u, 0u, 1u, 1u};
     if (P.fused && P.icld >= 1) {

@@ -34,7 +34,7 @@ cudaError_t upload_tables_fp32(const DevTables& t);
 // setcoef of the FP32 form (FP32 arithmetic, the FP64 form's indices) over all (column, layer)
 cudaError_t launch_setcoef_f32(const SolveParams& P, const float* tab, const double* tab64, float* cf, int* pk,
                                double* pdp, cudaStream_t s);
-// allow_tiled = false keeps the scratch-based kernel (k_solve<float>)
+// allow_tiled = false keeps the scratch-based kernel (k_solve)
 LaunchInfo plan_fp32(const SolveParams& P, int num_sms, bool allow_tiled = true);
 cudaError_t launch_solve_fp32(const SolveParams& P, const float* tab, const double* tab64, const LaunchInfo& li,
                               cudaStream_t s);

@@ -208,7 +208,7 @@ cudaError_t launch_setcoef_f32(const SolveParams& P, const float* tab, const dou
 cudaError_t upload_tables_fp32(const DevTables& t) { return cudaMemcpyToSymbol(cT, &t, sizeof(DevTables)); }
 
 // The tiled kernel's instance for a call: without aerosol a clear cell's
-// optics need a third fewer operations (262 144 x 60 with McICA clouds
+// optics need a third fewer operations (262 144 x 60 with icld 5
 // 105.7 -> 97.0 ms, 1024 x 60 clear 512 -> 495 us).
 static auto tiled_kernel(const SolveParams& P) { return P.iaer != 0 ? k_solve_tiled<true> : k_solve_tiled<false>; }
 

@@ -17,11 +17,12 @@ size_t slot_elems_fp64(const SolveParams& P, int nc) {
 }
 
 // Layers per CTA of the split kernels for a call that takes them, else 0.
-// They are the faster ones wherever they were measured (60 layers, clouds: 1
-// column 0.66 -> 0.17 ms, 63 x 47 1.02 -> 0.29, 304 1.29 -> 0.87, 608 1.81 ->
-// 1.54, 1 024 3.06 -> 2.65, 2 048 5.00 -> 4.55 ms), but they take one scratch slot
-// per column pair, so larger calls keep the fused kernel's one per resident
-// CTA.  The block of layers is the one whose CTAs fill the GPU's rounds of two
+// They are the faster ones below some 3 000 columns (60 layers, clouds, fused ->
+// split, whole calls: 1 column 0.57 -> 0.14 ms, 63 x 47 0.92 -> 0.26, 304 1.19 ->
+// 0.82, 608 1.68 -> 1.42, 1 024 2.62 -> 2.24, 2 048 4.68 -> 4.27, 2 432 5.29 -> 5.04,
+// 3 000 6.26 -> 6.23, 4 864 9.55 -> 9.83, 16 384 31.8 -> 32.7 ms), but they take one
+// scratch slot per column pair, so from 8 pairs per SM on (2 432 columns), or 2 GiB, calls
+// keep the fused kernel's one per resident CTA.  The block of layers is the one whose CTAs fill the GPU's rounds of two
 // CTAs per SM best, at one layer's time of preparation per CTA.
 static int split_layers(const SolveParams& P, int num_sms, size_t slot_bytes) {
     constexpr size_t kMaxScratch = (size_t)2 << 30;

@@ -44,7 +44,7 @@
 // (tile full / empty; per pair slot: pair produced, swept, finished) whose
 // waits give up after ~2^33 cycles with an error code instead of hanging.  A pair with more such cells than the
 // capacities below is listed for the caller, which solves it again with the
-// scratch-based kernel (k_solve<float>).
+// scratch-based kernel (k_solve).
 #pragma once
 
 #include "kernel.cuh"
@@ -587,7 +587,8 @@ __device__ void tiled_load(const SolveParams& P, const TCtx& X, int lp) {
 // once for the band's 2 to 12 subcolumns; those without a cloudy subcolumn
 // are left out (their inputs need not be valid).  Cloudy cells cost 40 % of a
 // call with McICA clouds, half of that for the optics each lane worked out for
-// itself: 262 144 x 60 113 -> 104 ms, 16 384 x 60 icld 5 6.4 -> 5.9 ms.
+// itself: 262 144 x 60 with icld 2 113 -> 104 ms, with icld 5 97 -> 88 ms,
+// 16 384 x 60 icld 5 6.4 -> 5.9 ms.
 __device__ void tiled_clouds(const SolveParams& P, const TCtx& X, int lp, const float* __restrict__ tab) {
     const TileView& V = X.V;
     const int L = X.L;
