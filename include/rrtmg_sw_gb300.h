@@ -178,7 +178,8 @@ int rrtmg_sw_nomcica_dev_c(const rrtmg_sw_args *a, const rrtmg_sw_clouds *c, voi
  * intermediates of each cell's layer solution from the forward pass (more
  * memory), 0 recomputes them in the reverse pass, -1 chooses by memory: stored when that scratch fits in half
  * of the free device memory; rrtmg_sw_last_ad_store_c reports the choice.
- * (rrtmg_sw_tl_c has no reverse pass: the same scratch and results either way.) */
+ * (rrtmg_sw_tl_c has no reverse pass: the same scratch and results either way.)
+ * Gradients and dJ differ in their last bits from run to run. */
 typedef struct rrtmg_sw_ad_args {
     double w_toa_up, w_sfc_net, w_hr_sum;
     int32_t store, pad;
